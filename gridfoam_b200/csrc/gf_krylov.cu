@@ -9,7 +9,7 @@
 // wait is bounded; on expiry the kernel raises an error flag and returns
 // instead of hanging.  The launch is cooperative, so all blocks are
 // co-resident and the barrier is always reachable.
-#include "gf_common.cuh"
+#include "gf_krylov.cuh"
 
 #include <cstdlib>
 #include <cstring>
@@ -75,17 +75,6 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
-__device__ __forceinline__ double nmax(double a, double b) {
-    if (a != a || b != b) return __longlong_as_double(0x7ff8000000000000LL);
-    return fmax(a, b);
-}
-
-__device__ __forceinline__ double inv_diag(const double* __restrict__ diag, int64_t c, bool jac) {
-    if (!jac) return 1.0;
-    const double d = __ldg(diag + c);
-    return fabs(d) < 2.220446049250313e-16 ? 1.0 : 1.0 / d;
-}
-
 // Grid-wide reduction of NV values per thread (sum, or max where maxmask
 // has the bit set), fused with the grid barrier.  Returns false when the
 // barrier wait expired or another block reported an error.  Every block
@@ -97,8 +86,6 @@ __device__ __forceinline__ double inv_diag(const double* __restrict__ diag, int6
 // counter barrier.
 constexpr int kW0Loads = 5;
 constexpr int kW0Blocks = 32 * kW0Loads;
-
-__device__ __forceinline__ double comb(double x, double y, bool mx) { return mx ? nmax(x, y) : x + y; }
 
 // Staging of the partials in grid_reduce_w0 (warp 0 only, between its wait
 // and the CTA barrier that ends the reduction).
@@ -427,12 +414,6 @@ __device__ __forceinline__ void row_apply(const gf_krylov_t& K, int64_t c, const
                 for (int k = 0; k < NC; ++k) out[k] += a[j] * g(k, nb[j]);
     }
 }
-
-__device__ __forceinline__ double norm_acc(double acc, double r, bool linf) {
-    return linf ? nmax(acc, fabs(r)) : acc + r * r;
-}
-
-__device__ __forceinline__ double norm_fin(double acc, bool linf) { return linf ? acc : sqrt(acc); }
 
 struct CgState {
     double thresh, r0, final, rz_old, alpha, beta;
@@ -3394,25 +3375,6 @@ static BoxVariant sr_box_kernel(int variant) {
     }
 }
 
-// BiCGStab per-component modes.
-enum { kDone = 0, kRun = 1, kRestart = 2, kIdle = 3, kConvS = 4 };
-
-struct BiState {
-    double thresh, r0, final, rho_old, alpha, omega, beta;
-    int mode, restarts, its, converged, status;
-};
-
-__device__ __forceinline__ void breakdown(BiState& s, int it, int max_restart) {
-    if (s.restarts >= max_restart) {
-        s.mode = kDone;
-        s.its = it;
-        s.status = GF_BREAKDOWN;
-    } else {
-        s.restarts += 1;
-        s.mode = kRestart;
-    }
-}
-
 // WIDTH: the ELL row width at compile time (6) or 0 (any).  The Jacobi
 // inverse of every cell is computed once per solve into the workspace (after
 // the six vectors) and gathered from there by the preconditioned SpMVs.
@@ -4753,8 +4715,6 @@ static int launch_split(const gf_krylov_t* k, void* stream, int which) {
 // blocks [blk0[i], blk0[i+1]) and runs the single-system kernel's body on
 // them with its own barrier counter and partials (its workspace), so its
 // iterates do not depend on which other systems share the launch.
-constexpr int kMaxBatch = 16;
-
 struct KBatch {
     int count;
     int blk0[kMaxBatch + 1];
@@ -5244,6 +5204,8 @@ int gf_pcg_solve(const gf_krylov_t* k, void* stream) {
                 const int st = launch_qrec(k, stream, k->variant == kQrecVariant ? 1 : 2);
                 if (st != GF_ERR_INVALID) return st;
             }
+            if (k->variant == kHaloVariant && cluster_fits(*k, false))
+                return launch_cluster(k, 1, false, false, reinterpret_cast<cudaStream_t>(stream));
             if (k->variant == kHaloVariant || k->variant == kHaloVariant + 1) {
                 const int st = launch_halo(k, stream, k->variant == kHaloVariant ? 1 : 2);
                 if (st != GF_ERR_INVALID) return st;
@@ -5309,6 +5271,7 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream) {
         }
     }
     if (!valid_krylov(k, 6, "gf_bicgstab_solve", k ? k->n : 0)) return GF_ERR_INVALID;
+    if (cluster_fits(*k, true)) return launch_cluster(k, 1, true, false, reinterpret_cast<cudaStream_t>(stream));
     const bool w6 = k->width == 6;
     switch (k->ncomp) {
         case 1:
@@ -5336,8 +5299,8 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
     }
     KBatch B;
     memset(&B, 0, sizeof(B));
-    B.count = count;
-    int total = 0;
+    gf_krylov_t small[kMaxBatch];
+    int nsmall = 0, total = 0, nblk = 0;
     for (int i = 0; i < count; ++i) {
         const gf_krylov_t& k = sys[i];
         if (k.mixed && bicg) {
@@ -5369,11 +5332,19 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
             set_error("%s: system %d: block count %d outside 1..%d", what, i, blocks[i], kMaxBlocks);
             return GF_ERR_INVALID;
         }
-        B.sys[i] = k;
-        B.blk0[i] = total;
         total += blocks[i];
+        // A system's route depends on itself alone, so its bits do not
+        // depend on the others: one cluster where it fits, else its share of
+        // the cooperative launch.
+        if (cluster_fits(k, bicg)) {
+            small[nsmall++] = k;
+            continue;
+        }
+        B.sys[B.count] = k;
+        B.blk0[B.count++] = nblk;
+        nblk += blocks[i];
     }
-    B.blk0[count] = total;
+    B.blk0[B.count] = nblk;
     const void* kern = !bicg ? (const void*)k_pcg1_batched
                              : (sys[0].ncomp == 1 ? (const void*)k_bicgstab_batched<1>
                                                   : sys[0].ncomp == 2 ? (const void*)k_bicgstab_batched<2>
@@ -5393,6 +5364,10 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
         return GF_ERR_INVALID;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    if (nsmall > 0) {
+        const int rc = launch_cluster(small, nsmall, bicg, true, st);
+        if (rc != GF_OK || B.count == 0) return rc;
+    }
     k_batch_reset<<<1, 32, 0, st>>>(B);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -5400,7 +5375,7 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
         return GF_ERR_CUDA;
     }
     void* args[] = {&B};
-    e = cudaLaunchCooperativeKernel(kern, dim3(total), dim3(threads), args, 0, st);
+    e = cudaLaunchCooperativeKernel(kern, dim3(nblk), dim3(threads), args, 0, st);
     if (e != cudaSuccess) {
         set_error("%s: cooperative launch failed: %s", what, cudaGetErrorString(e));
         return GF_ERR_CUDA;

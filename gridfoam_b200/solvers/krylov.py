@@ -49,8 +49,10 @@ def _split_graph_loop() -> bool:
 def default_variant(n: int, mixed: bool, symmetric: bool, box: bool = True) -> int:
     """CG launch shape by system size, from fixed-iteration timings on B200
     (``python -m gridfoam_b200.solvers.autotune``).  FP64 up to ~400K cells:
-    one grid reduction and a halo sync with the neighbouring blocks per
-    iteration, vectors in shared memory (6.9 against 9.8 us an iteration
+    one reduction per iteration, up to ~43K cells on one thread-block cluster
+    with everything on the chip (2.1 against 6.4 us an iteration at 16^3, 4.0
+    against 6.7 at 32^3), above that on the grid with a halo sync between
+    neighbouring blocks and the vectors in shared memory (6.9 against 9.8 us
     for 256-thread register blocks at 48^3, 8.0 against 8.2 for the
     q-recurrence form at 64^3); then, up to ~1.3M cells, the q-recurrence
     form (q = A z + beta q, z alone gathered; 14.7 us at 1M cells); above
