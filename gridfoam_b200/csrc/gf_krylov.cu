@@ -19,24 +19,8 @@ namespace gf {
 
 constexpr int kKThreads = 512;
 constexpr int kCgThreads = 256;
-constexpr int kMaxBlocks = 1024;
-constexpr int kMaxNV = 16;
-constexpr int kCtlDoubles = 32;
-constexpr long long kSpinLimit = 30000000LL;  // x ~40 ns polls: about a second
 // Slots of a runtime-width matrix row whose loads are issued together.
 constexpr int kSlotGroup = 8;
-
-// Partial sums are double-buffered by barrier parity: a block may write the
-// next barrier's partials while a slower block still reads this one's, but
-// not the one after (that needs the slow block's arrival).
-constexpr int64_t kPartials = 2LL * kMaxBlocks * kMaxNV;
-constexpr int64_t kHeader = kCtlDoubles + kPartials;
-
-struct KCtl {
-    unsigned long long count;  // barrier arrivals since launch (zeroed per launch)
-    int error;
-    int pad;
-};
 
 // Barriers this block has passed since the kernel started, and the poll
 // limit of every bounded wait of this launch; barrier_init() must run at the
@@ -59,20 +43,6 @@ __device__ __forceinline__ void barrier_init_v(const gf_krylov_t& K, int nblk, i
 
 __device__ __forceinline__ void barrier_init(const gf_krylov_t& K) {
     barrier_init_v(K, (int)gridDim.x, (int)blockIdx.x);
-}
-
-__device__ __forceinline__ int vload(const int* p) { return *(const volatile int*)p; }
-
-// Release-add / acquire-load pair of the grid barrier (the CTA barrier
-// before the add makes it cumulative over the whole block's writes).
-__device__ __forceinline__ void arrive_release(unsigned long long* p) {
-    asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(p) : "memory");
-}
-
-__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long* p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
 }
 
 // Grid-wide reduction of NV values per thread (sum, or max where maxmask
@@ -3375,331 +3345,6 @@ static BoxVariant sr_box_kernel(int variant) {
     }
 }
 
-// WIDTH: the ELL row width at compile time (6) or 0 (any).  The Jacobi
-// inverse of every cell is computed once per solve into the workspace (after
-// the six vectors) and gathered from there by the preconditioned SpMVs.
-template <int NC, int WIDTH>
-__device__ void bicgstab_body(const gf_krylov_t& K, int vb, int vn) {
-    __shared__ BiState st[NC];
-    __shared__ int s_any;
-    KCtl* ctl = reinterpret_cast<KCtl*>(K.work);
-    const int bk = vb >= 0 ? vb : (int)blockIdx.x;
-    const int nbk = vn >= 0 ? vn : (int)gridDim.x;
-    barrier_init_v(K, nbk, bk);
-    double* partials = K.work + kCtlDoubles;
-    double* vec = partials + kPartials;
-    const int64_t n = K.n;
-    double* r = vec;
-    double* rh = vec + NC * n;
-    double* p = vec + 2 * NC * n;
-    double* v = vec + 3 * NC * n;
-    double* s = vec + 4 * NC * n;
-    double* t = vec + 5 * NC * n;
-    double* inv = vec + 6 * NC * n;
-    double* x = K.x;
-    const bool jac = K.jacobi != 0, linf = K.norm_inf != 0;
-    const int64_t t0 = bk * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t stride = (int64_t)nbk * blockDim.x;
-    bool ok = true;
-
-    {  // r = b - A x; r_hat = p = r; |r|, r.r; the Jacobi inverse
-        double loc[2 * NC];
-#pragma unroll
-        for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
-        auto gx = [&](int k, int64_t i) { return __ldcg(x + k * n + i); };
-        for (int64_t c = t0; c < n; c += stride) {
-            __stcg(inv + c, inv_diag(K.diag, c, jac));
-            double ax[NC];
-            row_apply<NC, WIDTH>(K, c, gx, ax);
-#pragma unroll
-            for (int k = 0; k < NC; ++k) {
-                const double rk = __ldg(K.rhs + k * n + c) - ax[k];
-                __stcg(r + k * n + c, rk);
-                __stcg(rh + k * n + c, rk);
-                __stcg(p + k * n + c, rk);
-                loc[k] = norm_acc(loc[k], rk, linf);
-                loc[NC + k] += rk * rk;
-            }
-        }
-        ok = grid_reduce<2 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
-        if (threadIdx.x == 0) {
-            for (int k = 0; k < NC; ++k) {
-                BiState& b = st[k];
-                const double r0 = norm_fin(loc[k], linf);
-                b.r0 = r0;
-                b.final = r0;
-                b.thresh = fmax(K.atol, K.rtol * r0);
-                b.rho_old = loc[NC + k];
-                b.restarts = 0;
-                b.its = 0;
-                b.converged = 0;
-                b.status = GF_MAX_ITER;
-                b.mode = kRun;
-                if (r0 < b.thresh) {
-                    b.mode = kDone;
-                    b.converged = 1;
-                    b.status = GF_OK;
-                } else if (!isfinite(r0)) {
-                    b.mode = kDone;
-                    b.status = GF_NONFINITE;
-                }
-            }
-        }
-        __syncthreads();
-    }
-
-    for (int it = 1; ok && it <= K.max_iter; ++it) {
-        if (threadIdx.x == 0) {
-            int any = 0;
-            for (int k = 0; k < NC; ++k) {
-                if (st[k].mode == kIdle) st[k].mode = kRun;
-                any |= (st[k].mode == kRun);
-            }
-            s_any = any;
-        }
-        __syncthreads();
-        if (!s_any) break;
-
-        // P1: y = M p, v = A y; r_hat.v, |r_hat|^2, |v|^2
-        {
-            double loc[3 * NC];
-#pragma unroll
-            for (int j = 0; j < 3 * NC; ++j) loc[j] = 0.0;
-            auto gy = [&](int k, int64_t i) { return __ldcg(inv + i) * __ldcg(p + k * n + i); };
-            for (int64_t c = t0; c < n; c += stride) {
-                double av[NC];
-                row_apply<NC, WIDTH>(K, c, gy, av);
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    if (st[k].mode != kRun) continue;
-                    __stcg(v + k * n + c, av[k]);
-                    const double h = __ldcg(rh + k * n + c);
-                    loc[k] += h * av[k];
-                    loc[NC + k] += h * h;
-                    loc[2 * NC + k] += av[k] * av[k];
-                }
-            }
-            ok = grid_reduce<3 * NC>(ctl, partials, loc, 0u);
-            if (!ok) break;
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < NC; ++k) {
-                    BiState& b = st[k];
-                    if (b.mode != kRun) continue;
-                    const double da = loc[k];
-                    if (fabs(da) <= 1e-6 * sqrt(loc[NC + k]) * sqrt(loc[2 * NC + k]))
-                        breakdown(b, it, K.max_restart);
-                    else
-                        b.alpha = b.rho_old / da;
-                }
-            }
-            __syncthreads();
-        }
-        // P2: s = r - alpha v, |s|; restarting systems copy r and reduce r.r
-        {
-            double loc[2 * NC];
-#pragma unroll
-            for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
-            for (int64_t c = t0; c < n; c += stride) {
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const int md = st[k].mode;
-                    if (md == kRun) {
-                        const double sk = __ldcg(r + k * n + c) - st[k].alpha * __ldcg(v + k * n + c);
-                        __stcg(s + k * n + c, sk);
-                        loc[k] = norm_acc(loc[k], sk, linf);
-                    } else if (md == kRestart) {
-                        const double rk = __ldcg(r + k * n + c);
-                        __stcg(rh + k * n + c, rk);
-                        __stcg(p + k * n + c, rk);
-                        loc[NC + k] += rk * rk;
-                    }
-                }
-            }
-            ok = grid_reduce<2 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
-            if (!ok) break;
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < NC; ++k) {
-                    BiState& b = st[k];
-                    if (b.mode == kRestart) {
-                        b.rho_old = loc[NC + k];
-                        b.mode = kIdle;
-                    } else if (b.mode == kRun) {
-                        const double fin = norm_fin(loc[k], linf);
-                        b.final = fin;
-                        if (fin < b.thresh) {
-                            b.mode = kConvS;
-                            b.converged = 1;
-                            b.its = it;
-                            b.status = GF_OK;
-                        } else if (!isfinite(fin)) {
-                            b.mode = kDone;
-                            b.its = it;
-                            b.status = GF_NONFINITE;
-                        }
-                    }
-                }
-            }
-            __syncthreads();
-        }
-        // P3: converged-on-s systems take x += alpha y; others z = M s, t = A z
-        {
-            double loc[2 * NC];
-#pragma unroll
-            for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
-            auto gz = [&](int k, int64_t i) { return __ldcg(inv + i) * __ldcg(s + k * n + i); };
-            for (int64_t c = t0; c < n; c += stride) {
-                double at[NC];
-                row_apply<NC, WIDTH>(K, c, gz, at);
-                const double ic = __ldcg(inv + c);
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const int md = st[k].mode;
-                    if (md == kConvS) {
-                        const double y = ic * __ldcg(p + k * n + c);
-                        __stcg(x + k * n + c, __ldcg(x + k * n + c) + st[k].alpha * y);
-                    } else if (md == kRun) {
-                        __stcg(t + k * n + c, at[k]);
-                        loc[k] += at[k] * at[k];
-                        loc[NC + k] += at[k] * __ldcg(s + k * n + c);
-                    }
-                }
-            }
-            ok = grid_reduce<2 * NC>(ctl, partials, loc, 0u);
-            if (!ok) break;
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < NC; ++k) {
-                    BiState& b = st[k];
-                    if (b.mode == kConvS) {
-                        b.mode = kDone;
-                        continue;
-                    }
-                    if (b.mode != kRun) continue;
-                    const double dd = loc[k];
-                    const double tn = sqrt(loc[k]);
-                    if (fabs(dd) <= 1e-6 * tn * tn) {
-                        breakdown(b, it, K.max_restart);
-                        continue;
-                    }
-                    b.omega = loc[NC + k] / dd;
-                    if (fabs(b.omega) <= 1e-6) breakdown(b, it, K.max_restart);
-                }
-            }
-            __syncthreads();
-        }
-        // P4: x += alpha y + omega z, r = s - omega t; |r|, r_hat.r, |r_hat|^2, |r|^2
-        {
-            double loc[4 * NC];
-#pragma unroll
-            for (int j = 0; j < 4 * NC; ++j) loc[j] = 0.0;
-            for (int64_t c = t0; c < n; c += stride) {
-                const double ic = __ldcg(inv + c);
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const int md = st[k].mode;
-                    if (md == kRun) {
-                        const double sk = __ldcg(s + k * n + c);
-                        const double y = ic * __ldcg(p + k * n + c);
-                        const double z = ic * sk;
-                        __stcg(x + k * n + c, __ldcg(x + k * n + c) + st[k].alpha * y + st[k].omega * z);
-                        const double rk = sk - st[k].omega * __ldcg(t + k * n + c);
-                        __stcg(r + k * n + c, rk);
-                        const double h = __ldcg(rh + k * n + c);
-                        loc[k] = norm_acc(loc[k], rk, linf);
-                        loc[NC + k] += h * rk;
-                        loc[2 * NC + k] += h * h;
-                        loc[3 * NC + k] += rk * rk;
-                    } else if (md == kRestart) {
-                        const double rk = __ldcg(r + k * n + c);
-                        __stcg(rh + k * n + c, rk);
-                        __stcg(p + k * n + c, rk);
-                        loc[3 * NC + k] += rk * rk;
-                    }
-                }
-            }
-            ok = grid_reduce<4 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
-            if (!ok) break;
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < NC; ++k) {
-                    BiState& b = st[k];
-                    if (b.mode == kRestart) {
-                        b.rho_old = loc[3 * NC + k];
-                        b.mode = kIdle;
-                        continue;
-                    }
-                    if (b.mode != kRun) continue;
-                    const double fin = norm_fin(loc[k], linf);
-                    b.final = fin;
-                    if (fin < b.thresh) {
-                        b.mode = kDone;
-                        b.converged = 1;
-                        b.its = it;
-                        b.status = GF_OK;
-                        continue;
-                    }
-                    if (!isfinite(fin)) {
-                        b.mode = kDone;
-                        b.its = it;
-                        b.status = GF_NONFINITE;
-                        continue;
-                    }
-                    const double rho_new = loc[NC + k];
-                    if (fabs(rho_new) <= 1e-6 * sqrt(loc[2 * NC + k]) * sqrt(loc[3 * NC + k])) {
-                        breakdown(b, it, K.max_restart);
-                        continue;
-                    }
-                    b.beta = (rho_new / b.rho_old) * (b.alpha / b.omega);
-                    b.rho_old = rho_new;
-                }
-            }
-            __syncthreads();
-        }
-        // P5: p = r + beta (p - omega v); restarting systems copy r
-        {
-            double loc[NC];
-#pragma unroll
-            for (int k = 0; k < NC; ++k) loc[k] = 0.0;
-            for (int64_t c = t0; c < n; c += stride) {
-#pragma unroll
-                for (int k = 0; k < NC; ++k) {
-                    const int md = st[k].mode;
-                    if (md == kRun) {
-                        const double pk = __ldcg(p + k * n + c);
-                        __stcg(p + k * n + c,
-                               __ldcg(r + k * n + c) + st[k].beta * (pk - st[k].omega * __ldcg(v + k * n + c)));
-                    } else if (md == kRestart) {
-                        const double rk = __ldcg(r + k * n + c);
-                        __stcg(rh + k * n + c, rk);
-                        __stcg(p + k * n + c, rk);
-                        loc[k] += rk * rk;
-                    }
-                }
-            }
-            ok = grid_reduce<NC>(ctl, partials, loc, 0u);
-            if (!ok) break;
-            if (threadIdx.x == 0) {
-                for (int k = 0; k < NC; ++k) {
-                    if (st[k].mode == kRestart) {
-                        st[k].rho_old = loc[k];
-                        st[k].mode = kIdle;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (bk == 0 && threadIdx.x == 0) {
-        for (int k = 0; k < NC; ++k) {
-            double* o = K.stats + 5 * k;
-            const bool fin = st[k].mode == kDone;
-            o[0] = st[k].r0;
-            o[1] = st[k].final;
-            o[2] = fin ? st[k].its : K.max_iter;
-            o[3] = st[k].converged;
-            o[4] = ok ? (fin ? st[k].status : GF_MAX_ITER) : GF_ERR_TIMEOUT;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Mixed precision BiCGStab: FP32 inner BiCGStab cycles inside FP64
 // iterative refinement, for all NC components in one launch.  Each cycle
@@ -4715,18 +4360,6 @@ static int launch_split(const gf_krylov_t* k, void* stream, int which) {
 // blocks [blk0[i], blk0[i+1]) and runs the single-system kernel's body on
 // them with its own barrier counter and partials (its workspace), so its
 // iterates do not depend on which other systems share the launch.
-struct KBatch {
-    int count;
-    int blk0[kMaxBatch + 1];
-    gf_krylov_t sys[kMaxBatch];
-};
-
-__device__ __forceinline__ int batch_system(const KBatch& B) {
-    int s = 0;
-    while (s + 1 < B.count && (int)blockIdx.x >= B.blk0[s + 1]) ++s;
-    return s;
-}
-
 // Zeroes every system's barrier control block (one launch for the batch).
 __global__ void k_batch_reset(const KBatch B) {
     for (int i = threadIdx.x; i < B.count; i += blockDim.x) {
@@ -4775,22 +4408,6 @@ __global__ void __launch_bounds__(kCgThreads, 4) k_pcg1_batched(const KBatch B) 
         EllRows<double, 0> rows{K.val, K.nbr, K.n, K.width, K.row_len};
         pcg1_body<kCgThreads, 1>(K, rows, bid, nb);
     }
-}
-
-template <int NC>
-__global__ void __launch_bounds__(kKThreads) k_bicgstab_batched(const KBatch B) {
-    const int s = batch_system(B);
-    const gf_krylov_t& K = B.sys[s];
-    const int bid = (int)blockIdx.x - B.blk0[s], nb = B.blk0[s + 1] - B.blk0[s];
-    if (K.width == 6)
-        bicgstab_body<NC, 6>(K, bid, nb);
-    else
-        bicgstab_body<NC, 0>(K, bid, nb);
-}
-
-template <int NC, int WIDTH>
-__global__ void __launch_bounds__(kKThreads) k_bicgstab(gf_krylov_t K) {
-    bicgstab_body<NC, WIDTH>(K, -1, -1);
 }
 
 template <class Kern>
@@ -5271,19 +4888,12 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream) {
         }
     }
     if (!valid_krylov(k, 6, "gf_bicgstab_solve", k ? k->n : 0)) return GF_ERR_INVALID;
-    if (cluster_fits(*k, true)) return launch_cluster(k, 1, true, false, reinterpret_cast<cudaStream_t>(stream));
-    const bool w6 = k->width == 6;
-    switch (k->ncomp) {
-        case 1:
-            return w6 ? launch_persistent(k_bicgstab<1, 6>, k, stream, "gf_bicgstab_solve")
-                      : launch_persistent(k_bicgstab<1, 0>, k, stream, "gf_bicgstab_solve");
-        case 2:
-            return w6 ? launch_persistent(k_bicgstab<2, 6>, k, stream, "gf_bicgstab_solve")
-                      : launch_persistent(k_bicgstab<2, 0>, k, stream, "gf_bicgstab_solve");
-        default:
-            return w6 ? launch_persistent(k_bicgstab<3, 6>, k, stream, "gf_bicgstab_solve")
-                      : launch_persistent(k_bicgstab<3, 0>, k, stream, "gf_bicgstab_solve");
+    if (k->stride_y > 0 && (k->width != 6 || k->stride_z < k->stride_y)) {
+        set_error("gf_bicgstab_solve: a box layout needs width 6 and strides 1 <= stride_y <= stride_z");
+        return GF_ERR_INVALID;
     }
+    if (cluster_fits(*k, true)) return launch_cluster(k, 1, true, false, reinterpret_cast<cudaStream_t>(stream));
+    return launch_persistent(bicgstab_kernel(*k), k, stream, "gf_bicgstab_solve", kBicgThreads);
 }
 
 }  // extern "C"
@@ -5345,11 +4955,8 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
         nblk += blocks[i];
     }
     B.blk0[B.count] = nblk;
-    const void* kern = !bicg ? (const void*)k_pcg1_batched
-                             : (sys[0].ncomp == 1 ? (const void*)k_bicgstab_batched<1>
-                                                  : sys[0].ncomp == 2 ? (const void*)k_bicgstab_batched<2>
-                                                                      : (const void*)k_bicgstab_batched<3>);
-    const int threads = bicg ? kKThreads : kCgThreads;
+    const void* kern = bicg ? bicgstab_batched_kernel(sys[0].ncomp) : (const void*)k_pcg1_batched;
+    const int threads = bicg ? kBicgThreads : kCgThreads;
     int dev = 0, sms = 0, coop = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -5394,10 +5001,10 @@ int gf_bicgstab_solve_batched(const gf_krylov_t* systems, int32_t count, const i
 }
 
 int gf_batch_max_blocks(int32_t bicgstab) {
-    const void* kern = bicgstab ? (const void*)k_bicgstab_batched<3> : (const void*)k_pcg1_batched;
+    const void* kern = bicgstab ? bicgstab_batched_kernel(3) : (const void*)k_pcg1_batched;
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-        cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bicgstab ? kKThreads : kCgThreads,
+        cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bicgstab ? kBicgThreads : kCgThreads,
                                                                       0) != cudaSuccess) {
         set_error("gf_batch_max_blocks: device query failed");
         return -1;

@@ -7,6 +7,36 @@
 namespace gf {
 
 constexpr int kMaxBatch = 16;  // systems of a batched launch
+constexpr int kMaxBlocks = 1024;
+constexpr int kMaxNV = 16;
+constexpr int kCtlDoubles = 32;
+constexpr long long kSpinLimit = 30000000LL;  // x ~40 ns polls: about a second
+
+// Partial sums are double-buffered by barrier parity: a block may write the
+// next barrier's partials while a slower block still reads this one's, but
+// not the one after (that needs the slow block's arrival).
+constexpr int64_t kPartials = 2LL * kMaxBlocks * kMaxNV;
+constexpr int64_t kHeader = kCtlDoubles + kPartials;
+
+struct KCtl {
+    unsigned long long count;  // barrier arrivals since launch (zeroed per launch)
+    int error;
+    int pad;
+};
+
+__device__ __forceinline__ int vload(const int* p) { return *(const volatile int*)p; }
+
+// Release-add / acquire-load pair of the grid barrier (the CTA barrier
+// before the add makes it cumulative over the whole block's writes).
+__device__ __forceinline__ void arrive_release(unsigned long long* p) {
+    asm volatile("fence.acq_rel.gpu;\n\tred.relaxed.gpu.global.add.u64 [%0], 1;" ::"l"(p) : "memory");
+}
+
+__device__ __forceinline__ unsigned long long load_acquire(const unsigned long long* p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
 
 // Maximum that keeps a NaN (a norm with one must not pass a stopping test).
 __device__ __forceinline__ double nmax(double a, double b) {
@@ -46,6 +76,25 @@ __device__ __forceinline__ void breakdown(BiState& s, int it, int max_restart) {
         s.mode = kRestart;
     }
 }
+
+// The systems of a batched cooperative launch: system i owns the blocks
+// [blk0[i], blk0[i+1]).
+struct KBatch {
+    int count;
+    int blk0[kMaxBatch + 1];
+    gf_krylov_t sys[kMaxBatch];
+};
+
+__device__ __forceinline__ int batch_system(const KBatch& B) {
+    int s = 0;
+    while (s + 1 < B.count && (int)blockIdx.x >= B.blk0[s + 1]) ++s;
+    return s;
+}
+
+// Grid BiCGStab kernels (gf_bicgstab.cu).
+const void* bicgstab_kernel(const gf_krylov_t& k);
+const void* bicgstab_batched_kernel(int ncomp);
+constexpr int kBicgThreads = 1024;
 
 // Solves on one thread-block cluster a system (gf_cluster.cu).  The launch
 // functions return GF_ERR_INVALID without a launch when a system does not

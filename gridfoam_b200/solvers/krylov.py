@@ -204,9 +204,9 @@ class DeviceKrylov(LinearSolver):
         k.variant = (int(self.variant) if self.variant is not None
                      else default_variant(n, mixed, symmetric, box is not None))
         k.single_reduction = int(self.single_reduction and not mixed and not self.bicgstab and nc == 1)
-        if box is not None and not self.bicgstab and nc == 1:
+        if box is not None and (not mixed if self.bicgstab else nc == 1):
             k.stride_y, k.stride_z = box
-            k.symmetric = int(symmetric)
+            k.symmetric = int(symmetric and not self.bicgstab)
         return k, stats
 
     def _solve_matrix(self, A, rhs_store: torch.Tensor, x0_store: torch.Tensor) -> SolveResult:
