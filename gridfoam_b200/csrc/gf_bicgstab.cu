@@ -25,122 +25,22 @@
 // reductions of up to twelve values before it in brackets): 25.7 (57) on a
 // box of 147K cells, 80 (179) at 535K, 44 (80) on an octree of 236K, 265 at
 // 1.73M, 605 (1000) at 4.08M: 4.3 TB/s of the 640 bytes a cell.
-#include "gf_krylov.cuh"
+#include "gf_gridsync.cuh"
 
 namespace gf {
 
 namespace {
 
 constexpr int kT = kBicgThreads;
-constexpr int kBiValues = 9;
-constexpr int kBiLoads = 5;  // partials a lane reads at once: one block an SM, 148 of them
-constexpr int kBiSlots = kT / 2;  // per value in shared memory
 // Row forms: any ELL rows, rows of exactly six slots, and six slots with the
 // implicit neighbours of a uniform lexicographic box (the index table is not
 // read, and the gathers do not wait for it).
 enum { kEll = 0, kEll6 = 1, kBox = 2 };
 
-struct BiShared {
-    // barrier state of this block's system
-    unsigned epoch;
-    int nblk, bid, err;
-    long long spin;
-    // a reduction's totals and the threads' values
-    double total[kBiValues];
+struct BiShared : GridShared<kT, 9> {
     double hh[3];  // |r_hat|^2
     int restart;
-    double mine[kBiValues * kBiSlots];
 };
-
-// Arrive and wait for all blocks of the system (bounded; false: gave up, or
-// another block did).  The CTA barriers make the release cumulative over the
-// block's writes and order its later reads behind the acquire.
-__device__ __forceinline__ bool bi_barrier(BiShared& sh, KCtl* ctl) {
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        const unsigned ep = sh.epoch;
-        __syncwarp();
-        if (threadIdx.x == 0) arrive_release(&ctl->count);
-        const unsigned long long target = (unsigned long long)(ep + 1u) * (unsigned)sh.nblk;
-        int err = 0;
-        long long it = 0;
-        while (true) {
-            const unsigned long long c = load_acquire(&ctl->count);
-            if (__all_sync(0xffffffffu, c >= target)) break;
-            __nanosleep(20);
-            ++it;
-            if ((it & 255) == 0 && __any_sync(0xffffffffu, vload(&ctl->error) != 0)) {
-                err = 1;
-                break;
-            }
-            if (it > sh.spin) {
-                if (threadIdx.x == 0) atomicExch(&ctl->error, 1);
-                err = 1;
-                break;
-            }
-        }
-        if (threadIdx.x == 0) {
-            sh.err = err;
-            sh.epoch = ep + 1u;
-        }
-    }
-    __syncthreads();
-    return sh.err == 0;
-}
-
-// Sums over all blocks of NV values a thread (max where maxmask has the bit
-// set), and the barrier.  The totals are left in total; every block adds
-// the blocks' partials in the same fixed order.
-template <int NV>
-__device__ __forceinline__ bool bi_reduce(BiShared& sh, KCtl* ctl, double* partials, double (&v)[NV], unsigned maxmask) {
-    constexpr int kPer = kBiSlots / 32;
-    static_assert(NV <= kBiValues && 32 * NV <= kT, "one warp a value");
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // double-buffered by barrier parity (see kPartials)
-    double* part = partials + (sh.epoch & 1u) * (kPartials / 2);
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        v[j] = comb(v[j], __shfl_xor_sync(0xffffffffu, v[j], 16), (maxmask >> j) & 1u);
-        if (lane < 16) sh.mine[j * kBiSlots + warp * 16 + lane] = v[j];
-    }
-    __syncthreads();
-    const bool mx = (maxmask >> warp) & 1u;
-    if (warp < NV) {
-        double x[kPer];
-#pragma unroll
-        for (int k = 0; k < kPer; ++k) x[k] = sh.mine[warp * kBiSlots + k * 32 + lane];
-#pragma unroll
-        for (int h = kPer / 2; h > 0; h >>= 1)
-#pragma unroll
-            for (int k = 0; k < h; ++k) x[k] = comb(x[k], x[k + h], mx);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x[0] = comb(x[0], __shfl_xor_sync(0xffffffffu, x[0], o), mx);
-        if (lane == 0) __stcg(part + (int64_t)warp * kMaxBlocks + sh.bid, x[0]);
-    }
-    if (!bi_barrier(sh, ctl)) return false;
-    if (warp < NV) {
-        // Every load of a lane issued before any is added: in a plain loop the
-        // five L2 round trips follow one another (3.4 us a reduction of 148
-        // blocks against 2.1).
-        const int nblk = sh.nblk;
-        double x = 0.0;  // the identity of both: the max values are norms
-        for (int b0 = lane; b0 < nblk; b0 += 32 * kBiLoads) {
-            double y[kBiLoads];
-#pragma unroll
-            for (int q = 0; q < kBiLoads; ++q) {
-                const int b = b0 + 32 * q;
-                y[q] = b < nblk ? __ldcg(part + (int64_t)warp * kMaxBlocks + b) : 0.0;
-            }
-#pragma unroll
-            for (int q = 0; q < kBiLoads; ++q) x = comb(x, y[q], mx);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) x = comb(x, __shfl_xor_sync(0xffffffffu, x, o), mx);
-        if (lane == 0) sh.total[warp] = x;
-    }
-    __syncthreads();
-    return true;
-}
 
 // out_k = diag g(k, c) + sum_s val(s, c) g(k, nbr(s, c)), the loads of GRP
 // slots issued before their products.
@@ -185,13 +85,7 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
     // cells of a box); two at a time: 657.
     constexpr int GRP = NC > 1 ? 3 : 6;
     KCtl* ctl = reinterpret_cast<KCtl*>(K.work);
-    if (threadIdx.x == 0) {
-        sh.epoch = 0;
-        sh.nblk = nbk;
-        sh.bid = bk;
-        sh.err = 0;
-        sh.spin = K.spin_limit > 0 ? K.spin_limit : kSpinLimit;
-    }
+    grid_init(sh, K, nbk, bk);
     __syncthreads();
     double* partials = K.work + kCtlDoubles;
     double* vec = partials + kPartials;
@@ -229,7 +123,7 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
                 loc[NC + k] += rk * rk;
             }
         }
-        ok = bi_reduce<2 * NC>(sh, ctl, partials, loc, nmask);
+        ok = grid_sum<2 * NC>(sh, ctl, partials, loc, nmask);
         if (me < NC) {
             BiState& b = st[me];
             const double r0 = norm_fin(sh.total[me], linf);
@@ -291,7 +185,7 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
                     loc[NC + k] += av[k] * av[k];
                 }
             }
-            ok = bi_reduce<2 * NC>(sh, ctl, partials, loc, 0u);
+            ok = grid_sum<2 * NC>(sh, ctl, partials, loc, 0u);
             if (!ok) break;
             if (me < NC && st[me].mode == kRun) {
                 BiState& b = st[me];
@@ -306,7 +200,7 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
 #pragma unroll
             for (int k = 0; k < NC; ++k)
                 if (st[k].mode == kRun) s[k * n + c] = r[k * n + c] - st[k].alpha * v[k * n + c];
-        ok = bi_barrier(sh, ctl);
+        ok = grid_sync(sh, ctl);
         if (!ok) break;
         {  // P3 (and the restarts of P1's breakdowns)
             double loc[3 * NC];
@@ -330,7 +224,7 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
                     }
                 }
             }
-            ok = bi_reduce<3 * NC>(sh, ctl, partials, loc, nmask);
+            ok = grid_sum<3 * NC>(sh, ctl, partials, loc, nmask);
             if (!ok) break;
             if (me < NC) {
                 BiState& b = st[me];
@@ -388,12 +282,12 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
                 }
             }
             if (linf) {
-                ok = bi_reduce<3 * NC>(sh, ctl, partials, loc, nmask);
+                ok = grid_sum<3 * NC>(sh, ctl, partials, loc, nmask);
             } else {  // the 2-norm's own sum is |r|^2
                 double two[2 * NC];
 #pragma unroll
                 for (int j = 0; j < 2 * NC; ++j) two[j] = loc[j];
-                ok = bi_reduce<2 * NC>(sh, ctl, partials, two, 0u);
+                ok = grid_sum<2 * NC>(sh, ctl, partials, two, 0u);
             }
             if (!ok) break;
             if (threadIdx.x == 0) sh.restart = 0;
@@ -446,11 +340,11 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
                 }
             }
             if (sh.restart) {
-                ok = bi_reduce<NC>(sh, ctl, partials, loc, 0u);
+                ok = grid_sum<NC>(sh, ctl, partials, loc, 0u);
                 if (!ok) break;
                 if (me < NC && st[me].mode == kRestart) restarted(me);
             } else {
-                ok = bi_barrier(sh, ctl);
+                ok = grid_sync(sh, ctl);
             }
             __syncthreads();
         }

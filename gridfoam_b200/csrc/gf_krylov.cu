@@ -2431,12 +2431,6 @@ __global__ void __launch_bounds__(THREADS, MINB) k_pcg1_stream_ell(gf_krylov_t K
 // block keeps r, p, q and w of its cells in shared memory (4 doubles a
 // cell) and updates its cells of x in place in global memory.
 
-// Halo flags: one 64-bit epoch per block, one per 128-byte line (flags of
-// neighbouring blocks sharing a line cost ~1.7 us an iteration at 262K
-// cells), after z and the Jacobi inverse in the workspace.
-constexpr int64_t kHaloFlagStride = 16;
-constexpr int64_t kHaloFlagDoubles = kMaxBlocks * kHaloFlagStride;
-
 // Publish epoch ep for this block, then wait (bounded, like grid_reduce)
 // until blocks blo..bhi have published it.  The CTA barrier before the
 // release makes it cumulative over the whole block's writes; the acquires
@@ -4823,6 +4817,17 @@ int gf_pcg_solve(const gf_krylov_t* k, void* stream) {
             }
             if (k->variant == kHaloVariant && cluster_fits(*k, false))
                 return launch_cluster(k, 1, false, false, reinterpret_cast<cudaStream_t>(stream));
+            if (k->variant == kHaloVariant) {
+                int st = launch_resident(k, reinterpret_cast<cudaStream_t>(stream));
+                if (st != GF_ERR_INVALID) return st;
+                // Rows longer than six slots (octrees) beyond that: the
+                // q-recurrence form (16.0 us an iteration at 349K cells, the
+                // halo form 18.9; 12.6 against 15.0 at 236K).
+                if (!box && k->width > 6) {
+                    st = launch_qrec(k, stream, 1);
+                    if (st != GF_ERR_INVALID) return st;
+                }
+            }
             if (k->variant == kHaloVariant || k->variant == kHaloVariant + 1) {
                 const int st = launch_halo(k, stream, k->variant == kHaloVariant ? 1 : 2);
                 if (st != GF_ERR_INVALID) return st;

@@ -96,6 +96,16 @@ const void* bicgstab_kernel(const gf_krylov_t& k);
 const void* bicgstab_batched_kernel(int ncomp);
 constexpr int kBicgThreads = 1024;
 
+// Halo flags: one 64-bit epoch per block, one per 128-byte line (flags of
+// neighbouring blocks sharing a line cost ~1.7 us an iteration at 262K
+// cells), after z and the Jacobi inverse in the workspace.
+constexpr int64_t kHaloFlagStride = 16;
+constexpr int64_t kHaloFlagDoubles = kMaxBlocks * kHaloFlagStride;
+
+// CG with the system resident on the grid's SMs (gf_resident.cu);
+// GF_ERR_INVALID without a launch when it does not fit.
+int launch_resident(const gf_krylov_t* k, cudaStream_t st);
+
 // Solves on one thread-block cluster a system (gf_cluster.cu).  The launch
 // functions return GF_ERR_INVALID without a launch when a system does not
 // qualify; cluster_fits says so beforehand.

@@ -52,9 +52,9 @@ def default_variant(n: int, mixed: bool, symmetric: bool, box: bool = True) -> i
     one reduction per iteration, up to ~43K cells on one thread-block cluster
     with everything on the chip (2.1 against 6.4 us an iteration at 16^3, 4.0
     against 6.7 at 32^3), above that on the grid with a halo sync between
-    neighbouring blocks and the vectors in shared memory (6.9 against 9.8 us
-    for 256-thread register blocks at 48^3, 8.0 against 8.2 for the
-    q-recurrence form at 64^3); then, up to ~1.3M cells, the q-recurrence
+    neighbouring blocks, rows in shared memory and vectors in registers (6.1
+    us at 48^3 against 7.1 with the rows read again every iteration and 10.1
+    for 256-thread register blocks; 7.6 against 8.2 at 64^3); then, up to ~1.3M cells, the q-recurrence
     form (q = A z + beta q, z alone gathered; 14.7 us at 1M cells); above
     that the shared-memory tiled kernel for symmetric boxes, else the split
     CG (two plain kernels an iteration, variant 29).  FP32-inner (mixed) solves: 256-thread register
