@@ -3765,15 +3765,23 @@ __device__ __forceinline__ SplitScalars* split_scalars(const gf_krylov_t& K) {
 template <int NV>
 __device__ void split_sum(const double* part, int nblk, unsigned maxmask, double (&out)[NV]) {
     __shared__ double sh[NV][kSplitThreads / 32];
-    double acc[NV];
+    // Every load of a thread issued before any is added (a loop over nblk
+    // would wait for one L2 round trip after another).
+    constexpr int kPer = kMaxBlocks / kSplitThreads;
+    double y[NV][kPer], acc[NV];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) acc[j] = 0.0;
-    for (int b = threadIdx.x; b < nblk; b += blockDim.x)
+    for (int i = 0; i < kPer; ++i)
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            const double y = __ldcg(part + (int64_t)j * nblk + b);
-            acc[j] = ((maxmask >> j) & 1u) ? nmax(acc[j], y) : acc[j] + y;
+            const int b = threadIdx.x + i * kSplitThreads;
+            y[j][i] = b < nblk ? __ldcg(part + (int64_t)j * nblk + b) : 0.0;
         }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        acc[j] = 0.0;
+#pragma unroll
+        for (int i = 0; i < kPer; ++i) acc[j] = ((maxmask >> j) & 1u) ? nmax(acc[j], y[j][i]) : acc[j] + y[j][i];
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
@@ -4122,6 +4130,12 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_b(gf_krylov_t K, in
 // device), so the repeated solves of an algorithm reuse one instantiated
 // graph; the least recently used of kSplitLoops entries is replaced.
 constexpr int kSplitLoops = 64;
+// Iterations in the loop's body: testing the loop condition costs about as
+// much as a kernel boundary (1.73M-cell octree: 82.2 us an iteration with one
+// iteration a test and the partial sums loaded one after another, 78.7 with
+// four and all loads at once; 4.08M: 152.6 and 148.6).  The kernels of a body
+// after the solve has stopped return at once.
+constexpr int kSplitUnroll = 4;
 
 struct SplitLoop {
     int dev = -1;
@@ -4198,15 +4212,15 @@ static int split_loop_exec(const void* fa, const void* fb, const gf_krylov_t& K,
         ka.gridDim = dim3(grid);
         ka.blockDim = dim3(kSplitThreads);
         ka.kernelParams = a_args;
-        e = cudaGraphAddKernelNode(&na, body, nullptr, 0, &ka);
-        if (e == cudaSuccess) {
-            void* b_args[] = {&kcopy, &it0, &par0};
-            cudaKernelNodeParams kb = {};
-            kb.func = const_cast<void*>(fb);
-            kb.gridDim = dim3(grid);
-            kb.blockDim = dim3(kSplitThreads);
-            kb.kernelParams = b_args;
-            e = cudaGraphAddKernelNode(&nb, body, &na, 1, &kb);
+        void* b_args[] = {&kcopy, &it0, &par0};
+        cudaKernelNodeParams kb = {};
+        kb.func = const_cast<void*>(fb);
+        kb.gridDim = dim3(grid);
+        kb.blockDim = dim3(kSplitThreads);
+        kb.kernelParams = b_args;
+        for (int i = 0; i < kSplitUnroll && e == cudaSuccess; ++i) {
+            e = cudaGraphAddKernelNode(&na, body, i > 0 ? &nb : nullptr, i > 0 ? 1 : 0, &ka);
+            if (e == cudaSuccess) e = cudaGraphAddKernelNode(&nb, body, &na, 1, &kb);
         }
     }
     if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
