@@ -80,6 +80,14 @@ class GfMesh(ctypes.Structure):
         ("hang_move_n", P),
         ("face_axis", P),
         ("ell_len", P),
+        ("reg_level", P),
+        ("irr_cells", P),
+        ("hang_cells", P),
+        ("n_irr", I64),
+        ("n_hang_cells", I64),
+        ("reg_h", F64 * 3),
+        ("stride_y", I64),
+        ("stride_z", I64),
     ]
 
 
@@ -187,6 +195,7 @@ _SIGNATURES = {
     "gf_krylov_workspace_size": ([I64, I32, I32], I64),
     "gf_bc_state": ([P, P, P, P, P, P], ctypes.c_int),
     "gf_lsq_grad": ([P, I32, P, P, P, P, P], ctypes.c_int),
+    "gf_lsq_grad_hang": ([P, I32, P, P, P, P, P], ctypes.c_int),
     "gf_assemble": ([P, P, P], ctypes.c_int),
     "gf_momentum_finalize": ([P, I32, F64, P, P, P, P, P, P], ctypes.c_int),
     "gf_pressure_finalize": ([P, P, P, P, P, I64, F64, P], ctypes.c_int),

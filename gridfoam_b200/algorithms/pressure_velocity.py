@@ -126,7 +126,7 @@ class _PressureVelocity:
         # flux.py:132-162 correct_flux(phi, U, update_internal=True)
         self._eval_U()
         if self._hanging:
-            self._grad(self.U, self.grad_U)
+            self._grad_hang(self.U, self.grad_U)
         call("gf_face_flux", byref(g.cmesh), 0, ptr(self.U.store), ptr(self.U.table.kind),
              ptr(self.U.table.psib), None, ptr(self.grad_U) if self._hanging else None, ptr(self.phi.store),
              stream_ptr())
@@ -256,6 +256,13 @@ class _PressureVelocity:
         call("gf_lsq_grad", byref(self._grid.cmesh), field.num_components, ptr(field.store),
              ptr(t.kind), ptr(t.psib), ptr(out), stream_ptr())
 
+    def _grad_hang(self, field: CellField, out: torch.Tensor) -> None:
+        """The same at the cells with a hanging face only: all that the
+        hanging-face corrections read."""
+        t = field.table
+        call("gf_lsq_grad_hang", byref(self._grid.cmesh), field.num_components, ptr(field.store),
+             ptr(t.kind), ptr(t.psib), ptr(out), stream_ptr())
+
     def _grad_cfg(self, field: CellField, out: torch.Tensor, lsq: torch.Tensor) -> None:
         """The configured gradient into ``out`` (fv/schemes/grad.py): least
         squares, or Green-Gauss over the linear face values, whose hanging
@@ -280,7 +287,7 @@ class _PressureVelocity:
             # also fills grad_U (the hanging corrections') on a hanging mesh
             self._grad_cfg(self.U, self.grad_U_cfg, self.grad_U)
         elif self._hanging:
-            self._grad(self.U, self.grad_U)
+            self._grad_hang(self.U, self.grad_U)
         a = GfAssembly()
         a.ncomp = 3
         a.div_scheme = self._div_code
@@ -396,9 +403,7 @@ class _PressureVelocity:
         if self._hanging:
             # fvc.interpolate(HbyA): HbyA carries no boundary conditions, so
             # its least-squares gradient has internal equations only.
-            t = self.HbyA.table
-            call("gf_lsq_grad", byref(g.cmesh), 3, ptr(self.HbyA.store), ptr(t.kind), ptr(t.psib),
-                 ptr(self.grad_H), s)
+            self._grad_hang(self.HbyA, self.grad_H)
             grad_h = ptr(self.grad_H)
         call("gf_face_flux", byref(g.cmesh), 1, ptr(self.HbyA.store), ptr(self.U.table.kind),
              ptr(self.U.table.psib), None if d is None else byref(d), grad_h, ptr(self.phi_hbya.store), s)
@@ -446,7 +451,7 @@ class _PressureVelocity:
             a.val = ptr(self.pEqn.val)
             a.source = ptr(self.pEqn.source_store)
             if self._hanging:
-                self._grad(self.p, self.grad_p_lsq)
+                self._grad_hang(self.p, self.grad_p_lsq)
                 a.grad_lsq = ptr(self.grad_p_lsq)
                 a.lap_corrected = self._p_corrected
                 a.ffc = ptr(self.p_ffc)

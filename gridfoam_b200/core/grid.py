@@ -172,6 +172,8 @@ class AxisProjectedGrid:
         move_o[hidx, axis[hang_faces]] = 0.0
         move_n[hidx, axis[hang_faces]] = 0.0
 
+        reg_h, reg_level = self._regular_cells(centers, sizes, owner, neighbour, axis, d_all, immersed, dom_owner)
+
         # Boundary faces: domain | immersed upper | immersed lower
         iSf = Sf[imm_faces]
         i_mag = np.linalg.norm(iSf, axis=1) if Fi else np.zeros(0)
@@ -243,11 +245,34 @@ class AxisProjectedGrid:
         normals = getattr(ap, "anchor_normal", None)
         host.extra["anchor_normal"] = (np.asarray(normals, dtype=np.float64).reshape(Fi, 3)
                                        if normals is not None else None)
+        host.extra["reg_h"] = reg_h
+        host.extra["reg_level"] = reg_level
+        host.extra["hang_cells"] = np.unique(np.concatenate([owner[hang_faces], neighbour[hang_faces]]))
         host.extra["hang_faces"] = hang_faces
         host.extra["hang_offset"] = hang_offset
         host.extra["hang_move_o"] = move_o
         host.extra["hang_move_n"] = move_n
         return host
+
+    @staticmethod
+    def _regular_cells(centers, sizes, owner, neighbour, axis, d_all, immersed, dom_owner):
+        """``(h [3], level [C] uint8)``: cells whose six faces are internal,
+        not immersed and lead to cells of their own size ``h 2^level`` at
+        that distance along the axes; 255 for the others.  Their geometry
+        follows from the level, so the kernels need not read it."""
+        C = sizes.shape[0]
+        h = sizes.min(axis=0)
+        level = np.rint(np.log2(sizes[:, 0] / h[0]))
+        ok = (level < 32) & (sizes == h * np.exp2(level)[:, None]).all(axis=1)
+        fidx = np.arange(owner.shape[0])
+        d_n = np.abs(d_all[fidx, axis])
+        want = h[axis] * np.exp2(level[owner])
+        same = (ok[owner] & ok[neighbour] & (level[owner] == level[neighbour]) & ~immersed
+                & (np.abs(d_n - want) <= 1e-9 * want) & (np.abs(d_all).sum(axis=1) - d_n <= 1e-9 * want))
+        faces = np.bincount(owner, minlength=C) + np.bincount(neighbour, minlength=C)
+        faces += np.bincount(dom_owner, minlength=C)
+        regular = np.bincount(owner[same], minlength=C) + np.bincount(neighbour[same], minlength=C)
+        return h, np.where(ok & (faces == 6) & (regular == 6), level, 255).astype(np.uint8)
 
     def _build_ell(self) -> None:
         """Cell-centric slot table sorted by (cell, direction, face).
@@ -366,10 +391,13 @@ class AxisProjectedGrid:
             "face_pos_neigh": i32(h.extra["face_pos_neigh"]),
             "face_axis": torch.as_tensor(np.ascontiguousarray(h.axis, dtype=np.int8), device=dev),
         }
+        t["reg_level"] = torch.as_tensor(h.extra["reg_level"], device=dev)
+        t["irr_cells"] = i32(np.nonzero(h.extra["reg_level"] == 255)[0])
         hf = h.extra["hang_faces"]
         face_hang = np.full(self._num_internal_faces, -1, dtype=np.int64)
         face_hang[hf] = np.arange(hf.shape[0])
         if hf.shape[0]:
+            t["hang_cells"] = i32(h.extra["hang_cells"])
             t["hang_face"] = i32(hf)
             t["face_hang"] = i32(face_hang)
             t["hang_offset"] = f64(h.extra["hang_offset"].T)
@@ -384,6 +412,11 @@ class AxisProjectedGrid:
         m.n_bnd = self.num_bnd
         m.ell_width = self._ell_width
         m.n_hang = int(hf.shape[0])
+        m.n_irr = int(t["irr_cells"].numel())
+        m.n_hang_cells = int(h.extra["hang_cells"].shape[0])
+        m.reg_h = tuple(float(v) for v in h.extra["reg_h"])
+        if self.box_strides is not None:
+            m.stride_y, m.stride_z = self.box_strides
         for name, tensor in t.items():
             setattr(m, name, ptr(tensor))
         self.cmesh = m

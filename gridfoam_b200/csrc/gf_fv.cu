@@ -25,26 +25,30 @@ void set_error(const char* fmt, ...) {
 // ---------------------------------------------------------------------------
 // Boundary states (fv/boundary_ops.py:311-326, boundaries/**)
 // ---------------------------------------------------------------------------
-__global__ void k_bc_state(gf_mesh_t m, gf_bc_t bc, const double* __restrict__ psi,
-                           gf_bc_aux_t aux, gf_bc_state_t out) {
+template <int nc>
+__global__ void __launch_bounds__(128) k_bc_state(gf_mesh_t m, gf_bc_t bc, const double* __restrict__ psi,
+                                                  gf_bc_aux_t aux, gf_bc_state_t out) {
     const int64_t nb = m.n_bnd;
     const int64_t C = m.n_cells;
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb;
          b += (int64_t)gridDim.x * blockDim.x) {
         const int c = __ldg(m.bnd_cell + b);
         const int kind = bc.kind[b];
-        const int nc = bc.ncomp;
         const double mag_d = __ldg(m.bnd_mag_d + b);
-        double psiP[3], refv[3] = {0, 0, 0}, refg[3] = {0, 0, 0};
-        for (int k = 0; k < nc; ++k) psiP[k] = psi[k * C + c];
+        double psiP[3], value[3], refv[3] = {0, 0, 0}, refg[3] = {0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < nc; ++k) {
+            value[k] = __ldg(bc.value + k * nb + b);
+            psiP[k] = psi[k * C + c];
+        }
         double frac = 0.0;
         switch (kind) {
             case GF_BC_DIRICHLET:
                 frac = 1.0;
-                for (int k = 0; k < nc; ++k) refv[k] = bc.value[k * nb + b];
+                for (int k = 0; k < nc; ++k) refv[k] = value[k];
                 break;
             case GF_BC_NEUMANN:
-                for (int k = 0; k < nc; ++k) refg[k] = bc.value[k * nb + b];
+                for (int k = 0; k < nc; ++k) refg[k] = value[k];
                 break;
             case GF_BC_SLIP:
                 if (nc == 3) {
@@ -60,7 +64,7 @@ __global__ void k_bc_state(gf_mesh_t m, gf_bc_t bc, const double* __restrict__ p
             case GF_BC_INLET_OUTLET:
                 if (aux.phi_bnd != nullptr && aux.phi_bnd[b] < 0.0) {
                     frac = 1.0;
-                    for (int k = 0; k < nc; ++k) refv[k] = bc.value[k * nb + b];
+                    for (int k = 0; k < nc; ++k) refv[k] = value[k];
                 }
                 break;
             case GF_BC_FIXED_FLUX_P:
@@ -87,6 +91,7 @@ __global__ void k_bc_state(gf_mesh_t m, gf_bc_t bc, const double* __restrict__ p
                 break;
         }
         out.frac[b] = frac;
+#pragma unroll
         for (int k = 0; k < nc; ++k) {
             out.refv[k * nb + b] = refv[k];
             out.refg[k * nb + b] = refg[k];
@@ -376,6 +381,117 @@ __global__ void __launch_bounds__(256, NC == 1 ? 3 : 2) k_lsq_grad12(gf_mesh_t m
             }
         }
     }
+}
+
+// Gradient at cell c, any row, with the staged slots of k_lsq_grad12 (any
+// width; a row's used slots come first).
+template <int NC>
+__device__ __forceinline__ void lsq_any_cell(const gf_mesh_t& m, int64_t c, const double* __restrict__ psi,
+                                             const int8_t* __restrict__ kind, const double* __restrict__ psib,
+                                             double* __restrict__ grad) {
+    const int64_t C = m.n_cells;
+    const int W = m.ell_width;
+    double atb[NC][3], pc[NC];
+    const double cc[3] = {__ldg(m.center + c), __ldg(m.center + C + c), __ldg(m.center + 2 * C + c)};
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+        atb[k][0] = atb[k][1] = atb[k][2] = 0.0;
+        pc[k] = psi[k * C + c];
+    }
+    constexpr int G = 3;
+    for (int s0 = 0; s0 < W; s0 += G) {
+        if (s0 >= 6 && __ldg(m.ell_code + s0 * C + c) < 0) break;
+        lsq_slots<NC, G>(m, c, s0, W, psi, kind, psib, cc, pc, atb);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        double inv[3];
+#pragma unroll
+        for (int b = 0; b < 3; ++b) inv[b] = __ldg(m.lsq_ata_inv + (a * 3 + b) * C + c);
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+            grad[(k * 3 + a) * C + c] = inv[0] * atb[k][0] + inv[1] * atb[k][1] + inv[2] * atb[k][2];
+    }
+}
+
+// Gradient of the regular cells (mesh reg_level): six neighbours of the
+// cell's own size at distance h along the axes, so w2 d dT sums to twice the
+// identity and grad_a = (psi_+ - psi_-) / 2h, formed from the two differences
+// as in the other kernels.  The neighbours are implicit on a box (BOX), six
+// indices otherwise; neither slot codes nor centres nor the normal matrix are
+// read: 97 bytes a cell for three components on a box and 121 on an octree
+// against 290.  Measured, three components: 17 us on a 96^3 box (k_lsq_grad6 70),
+// 63 us on a 4.08M-cell octree (k_lsq_grad12 359), 7.8 TB/s of these bytes with
+// the neighbours in L2.  The other cells follow in k_lsq_list: in one launch
+// with these they cost the streaming its occupancy (123 us together on that
+// octree).
+template <int NC, bool BOX>
+__global__ void __launch_bounds__(256) k_lsq_regular(gf_mesh_t m, double3 inv_h, const double* __restrict__ psi,
+                                                     double* __restrict__ grad) {
+    const int64_t C = m.n_cells;
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= C) return;
+    const int level = __ldg(m.reg_level + c);
+    if (level == 255) return;
+    int64_t j[6];
+    if constexpr (BOX) {
+        const int64_t st[3] = {1, m.stride_y, m.stride_z};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            j[2 * a] = c - st[a];
+            j[2 * a + 1] = c + st[a];
+        }
+    } else {
+#pragma unroll
+        for (int s = 0; s < 6; ++s) j[s] = __ldg(m.ell_nbr + s * C + c);
+    }
+    double p[NC], pn[NC][6];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+        p[k] = __ldg(psi + k * C + c);
+#pragma unroll
+        for (int s = 0; s < 6; ++s) pn[k][s] = __ldg(psi + k * C + j[s]);
+    }
+    // 1 / 2h = (1 / reg_h) 2^-(level + 1), the power of two exact
+    const double scale = __longlong_as_double((1022LL - level) << 52);
+    const double ih[3] = {inv_h.x * scale, inv_h.y * scale, inv_h.z * scale};
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+#pragma unroll
+        for (int k = 0; k < NC; ++k)
+            grad[(k * 3 + a) * C + c] = ((pn[k][2 * a + 1] - p[k]) - (pn[k][2 * a] - p[k])) * ih[a];
+}
+
+// Gradient at the listed cells, one a thread: scattered, so bound by the
+// sectors they touch (about 80 of 32 bytes a cell for three components: 27 us
+// for the 54K boundary cells of a 96^3 box), not by the staging of the slots
+// (groups of six: the same time).
+constexpr int kLsqThreads = 128;
+
+template <int NC>
+__global__ void __launch_bounds__(kLsqThreads) k_lsq_list(gf_mesh_t m, int64_t n, const int32_t* __restrict__ cells,
+                                                          const double* __restrict__ psi,
+                                                          const int8_t* __restrict__ kind,
+                                                          const double* __restrict__ psib,
+                                                          double* __restrict__ grad) {
+    const int64_t i = blockIdx.x * (int64_t)kLsqThreads + threadIdx.x;
+    if (i < n) lsq_any_cell<NC>(m, __ldg(cells + i), psi, kind, psib, grad);
+}
+
+// Cells from which the regular cells get a kernel of their own.
+constexpr int64_t kRegularCells = 32768;
+
+static bool has_regular(const gf_mesh_t* m) {
+    return m->reg_level != nullptr && (m->irr_cells != nullptr || m->n_irr == 0) && m->n_cells >= kRegularCells &&
+           m->ell_width >= 6 && m->n_faces < (int64_t)INT32_MAX && m->reg_h[0] > 0.0 && m->reg_h[1] > 0.0 &&
+           m->reg_h[2] > 0.0;
+}
+
+static void lsq_list(const gf_mesh_t* m, int nc, int64_t n, const int32_t* cells, const double* psi,
+                     const int8_t* kind, const double* psib, double* grad, cudaStream_t st) {
+    if (n <= 0) return;
+    auto kern = nc == 1 ? k_lsq_list<1> : k_lsq_list<3>;
+    kern<<<grid_for(n, kLsqThreads), kLsqThreads, 0, st>>>(*m, n, cells, psi, kind, psib, grad);
 }
 
 // ---------------------------------------------------------------------------
@@ -939,20 +1055,36 @@ __global__ void k_momentum_finalize(int64_t C, int nc, double relax, const doubl
     }
 }
 
-// Face sum of a face field for cell c (fv/fvc/div.py:33-64, before / V).
+// Face sum of a face field for cell c (fv/fvc/div.py:33-64, before / V), six
+// slots at a time: their codes, the immersed ordinals (not for a regular
+// cell, mesh reg_level, and not without immersed faces), then their values,
+// without a branch between (with one, two of three warps of a box take the
+// chain of look-ups for their boundary cells).  Divergence on a 96^3 box: 31 ->
+// 20 us, on a 4.08M-cell octree 192 -> 110.
 __device__ __forceinline__ double face_sum(const gf_mesh_t& m, int64_t c, const double* __restrict__ phi) {
     const int64_t C = m.n_cells;
-    const int64_t F = m.n_faces;
+    const int F = (int)m.n_faces, W = m.ell_width;
+    const bool regular = m.reg_level != nullptr && __ldg(m.reg_level + c) != 255;
+    const bool look = m.n_imm > 0 && m.imm_index != nullptr && !regular;
     double sum = 0.0;
-    for (int s = 0; s < m.ell_width; ++s) {
-        const int32_t code = __ldg(m.ell_code + s * C + c);
-        const Slot sl = decode_slot(m, code);
-        if (sl.kind == kInternal) {
-            const double v = phi[sl.face];
-            sum += sl.side ? -v : v;
-        } else if (sl.kind == kBoundary) {
-            sum += phi[F + sl.bnd];
+    for (int s0 = 0; s0 < W; s0 += 6) {
+        int code[6], row[6];
+        // a row's used slots come first, and a regular cell has six
+        if (s0 > 0 && (regular || __ldg(m.ell_code + s0 * C + c) < 0)) break;
+#pragma unroll
+        for (int s = 0; s < 6; ++s) code[s] = s0 + s < W ? __ldg(m.ell_code + (s0 + s) * C + c) : -1;
+#pragma unroll
+        for (int s = 0; s < 6; ++s) {
+            row[s] = code[s] < 0 ? 0 : code[s] >> 1;
+            const int imm = look && code[s] >= 0 && row[s] < F ? __ldg(m.imm_index + row[s]) : -1;
+            if (imm >= 0) row[s] = F + (int)m.n_domain + ((code[s] & 1) ? (int)m.n_imm : 0) + imm;
         }
+        double v[6];
+#pragma unroll
+        for (int s = 0; s < 6; ++s) v[s] = code[s] >= 0 ? __ldg(phi + row[s]) : 0.0;
+#pragma unroll
+        for (int s = 0; s < 6; ++s)
+            if (code[s] >= 0) sum += (row[s] < F && (code[s] & 1)) ? -v[s] : v[s];
     }
     return sum;
 }
@@ -1265,21 +1397,24 @@ __global__ void k_face_flux(gf_mesh_t m, int mode, const double* __restrict__ ve
     }
 }
 
-// Internal faces of an axis-aligned grid without hanging faces
-// (face_axis given, no gradient correction): the arithmetic of k_face_flux
-// for the one non-zero Sf component, two faces per thread per pass with
-// every load of both faces issued before the loads that depend on them
-// (indices, then gathers), and no branch between the two levels.
-template <bool DDT>
-__global__ void __launch_bounds__(256, 3) k_face_flux_axis(gf_mesh_t m, const double* __restrict__ vel,
-                                                        gf_ddtcorr_t ddt, double* __restrict__ phi) {
+// Internal faces of an axis-aligned grid (face_axis given): the arithmetic of
+// k_face_flux for the one non-zero Sf component, two faces per thread per
+// pass with every load of both faces issued before the loads that depend on
+// them (indices, then gathers), and no branch between the two levels.  HANG:
+// the offset correction of the few hanging faces, with the gradient grad
+// (4.08M-cell octree: 111 us, k_face_flux 211).
+template <bool DDT, bool HANG>
+__global__ void __launch_bounds__(256, DDT ? 3 : 4) k_face_flux_axis(gf_mesh_t m, const double* __restrict__ vel,
+                                                                     gf_ddtcorr_t ddt,
+                                                                     const double* __restrict__ grad,
+                                                                     double* __restrict__ phi) {
     constexpr int U = 2;
     const int64_t C = m.n_cells;
     const int F = (int)m.n_faces;
     const int stride = gridDim.x * blockDim.x;
     const bool older = DDT && ddt.c != 0.0;
     for (int f0 = blockIdx.x * blockDim.x + threadIdx.x; f0 < F; f0 += U * stride) {
-        int f[U], o[U], n[U], ax[U], imm[U];
+        int f[U], o[U], n[U], ax[U], imm[U], hg[U];
         double w[U], p0[U], p00[U];
 #pragma unroll
         for (int u = 0; u < U; ++u) {
@@ -1289,7 +1424,8 @@ __global__ void __launch_bounds__(256, 3) k_face_flux_axis(gf_mesh_t m, const do
             n[u] = __ldg(m.neighbour + g);
             w[u] = __ldg(m.weight + g);
             ax[u] = __ldg(m.face_axis + g);
-            imm[u] = m.imm_index ? __ldg(m.imm_index + g) : -1;
+            imm[u] = m.n_imm > 0 && m.imm_index ? __ldg(m.imm_index + g) : -1;
+            hg[u] = HANG ? hang_of(m, g) : -1;
             if (DDT) {
                 p0[u] = __ldg(ddt.phi_old + g);
                 p00[u] = older ? __ldg(ddt.phi_older + g) : 0.0;
@@ -1318,7 +1454,8 @@ __global__ void __launch_bounds__(256, 3) k_face_flux_axis(gf_mesh_t m, const do
         for (int u = 0; u < U; ++u) {
             if (f[u] >= F) continue;
             double flux = 0.0;
-            const double vf = w[u] * vo[u] + (1.0 - w[u]) * vn[u];
+            double vf = w[u] * vo[u] + (1.0 - w[u]) * vn[u];
+            if (HANG && hg[u] >= 0) vf = vf + hang_value_corr(m, grad, ax[u], o[u], n[u], w[u], hg[u]);
             flux += vf * sfa[u];
             if (DDT) {
                 double u0f_sf = 0.0;
@@ -1340,67 +1477,114 @@ __global__ void __launch_bounds__(256, 3) k_face_flux_axis(gf_mesh_t m, const do
     }
 }
 
-__global__ void k_interpolate(gf_mesh_t m, int nc, const double* __restrict__ psi,
-                              const int8_t* __restrict__ kind, const double* __restrict__ psib,
-                              const double* __restrict__ grad, double* __restrict__ out) {
+// Two rows of the extended face layout a thread and pass: their indices,
+// then every gather, before any is used (one row at a time with a loop over
+// the components was a chain of dependent loads at 2.7-2.9 TB/s).  4.08M-cell
+// octree: interpolation of three components 272 -> 186 us (of 112 at the copy
+// rate), normal gradient of one 199 -> 108 (of 60).
+constexpr int kFaceRows = 2;
+
+struct FaceRow {
+    int64_t i;
+    int o, n, h;
+    bool internal, imm;
+};
+
+// Rows i, i + blockDim.x of a thread; h: the hanging ordinal where asked for.
+__device__ __forceinline__ void face_rows(const gf_mesh_t& m, bool hang, FaceRow (&r)[kFaceRows]) {
+    const int64_t F = m.n_faces;
+#pragma unroll
+    for (int u = 0; u < kFaceRows; ++u) {
+        r[u].i = (blockIdx.x * (int64_t)kFaceRows + u) * blockDim.x + threadIdx.x;
+        r[u].internal = r[u].i < F;
+        const int64_t f = r[u].internal ? r[u].i : 0;  // read in place of what is not there
+        r[u].o = F > 0 ? __ldg(m.owner + f) : 0;
+        r[u].n = F > 0 ? __ldg(m.neighbour + f) : 0;
+        r[u].imm = F > 0 && m.n_imm > 0 && m.imm_index && __ldg(m.imm_index + f) >= 0;
+        r[u].h = hang && F > 0 ? hang_of(m, (int)f) : -1;
+    }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(256) k_interpolate(gf_mesh_t m, const double* __restrict__ psi,
+                                                     const int8_t* __restrict__ kind,
+                                                     const double* __restrict__ psib,
+                                                     const double* __restrict__ grad, double* __restrict__ out) {
     const int64_t C = m.n_cells;
     const int64_t F = m.n_faces;
     const int64_t nb = m.n_bnd;
     const int64_t total = F + nb;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (i < F) {
-            const int f = (int)i;
-            const bool imm = m.imm_index && __ldg(m.imm_index + f) >= 0;
-            const int o = __ldg(m.owner + f), n = __ldg(m.neighbour + f);
-            const double w = __ldg(m.weight + f);
-            const int h = (grad && !imm) ? hang_of(m, f) : -1;
-            for (int k = 0; k < nc; ++k) {
-                double v = imm ? 0.0 : w * psi[k * C + o] + (1.0 - w) * psi[k * C + n];
-                if (h >= 0) v = v + hang_value_corr(m, grad, k, o, n, w, h);
-                out[k * total + f] = v;
+    FaceRow r[kFaceRows];
+    face_rows(m, grad != nullptr, r);
+    double w[kFaceRows], po[kFaceRows][NC], pn[kFaceRows][NC];
+#pragma unroll
+    for (int u = 0; u < kFaceRows; ++u) {
+        w[u] = F > 0 ? __ldg(m.weight + (r[u].internal ? r[u].i : 0)) : 0.0;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            po[u][k] = __ldg(psi + k * C + r[u].o);
+            pn[u][k] = __ldg(psi + k * C + r[u].n);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kFaceRows; ++u) {
+        if (r[u].internal) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                double v = r[u].imm ? 0.0 : w[u] * po[u][k] + (1.0 - w[u]) * pn[u][k];
+                if (r[u].h >= 0 && !r[u].imm) v = v + hang_value_corr(m, grad, k, r[u].o, r[u].n, w[u], r[u].h);
+                out[k * total + r[u].i] = v;
             }
-        } else {
-            const int b = (int)(i - F);
+        } else if (r[u].i < total) {
+            const int b = (int)(r[u].i - F);
             const int c = __ldg(m.bnd_cell + b);
             const bool cov = kind && kind[b] != GF_BC_NONE;
-            for (int k = 0; k < nc; ++k) out[k * total + i] = cov ? psib[k * nb + b] : psi[k * C + c];
+#pragma unroll
+            for (int k = 0; k < NC; ++k) out[k * total + r[u].i] = cov ? psib[k * nb + b] : psi[k * C + c];
         }
     }
 }
 
-__global__ void k_sn_grad(gf_mesh_t m, int nc, const double* __restrict__ psi, const int8_t* __restrict__ kind,
-                          const double* __restrict__ frac, const double* __restrict__ refv,
-                          const double* __restrict__ refg, const double* __restrict__ grad,
-                          double* __restrict__ out) {
+template <int NC>
+__global__ void __launch_bounds__(256) k_sn_grad(gf_mesh_t m, const double* __restrict__ psi,
+                                                 const int8_t* __restrict__ kind, const double* __restrict__ frac,
+                                                 const double* __restrict__ refv, const double* __restrict__ refg,
+                                                 const double* __restrict__ grad, double* __restrict__ out) {
     const int64_t C = m.n_cells;
     const int64_t F = m.n_faces;
     const int64_t nb = m.n_bnd;
     const int64_t total = F + nb;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total;
-         i += (int64_t)gridDim.x * blockDim.x) {
-        if (i < F) {
-            const int f = (int)i;
-            const bool imm = m.imm_index && __ldg(m.imm_index + f) >= 0;
-            const int o = __ldg(m.owner + f), n = __ldg(m.neighbour + f);
-            const double dc = __ldg(m.delta + f);
-            const int h = (grad && !imm) ? hang_of(m, f) : -1;
-            for (int k = 0; k < nc; ++k) {
-                double v = imm ? 0.0 : dc * (psi[k * C + n] - psi[k * C + o]);
-                if (h >= 0) v = v + hang_sn_corr(m, grad, k, o, n, dc, h);
-                out[k * total + f] = v;
+    FaceRow r[kFaceRows];
+    face_rows(m, grad != nullptr, r);
+    double dc[kFaceRows], po[kFaceRows][NC], pn[kFaceRows][NC];
+#pragma unroll
+    for (int u = 0; u < kFaceRows; ++u) {
+        dc[u] = F > 0 ? __ldg(m.delta + (r[u].internal ? r[u].i : 0)) : 0.0;
+#pragma unroll
+        for (int k = 0; k < NC; ++k) {
+            po[u][k] = __ldg(psi + k * C + r[u].o);
+            pn[u][k] = __ldg(psi + k * C + r[u].n);
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < kFaceRows; ++u) {
+        if (r[u].internal) {
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                double v = r[u].imm ? 0.0 : dc[u] * (pn[u][k] - po[u][k]);
+                if (r[u].h >= 0 && !r[u].imm) v = v + hang_sn_corr(m, grad, k, r[u].o, r[u].n, dc[u], r[u].h);
+                out[k * total + r[u].i] = v;
             }
-        } else {
-            const int b = (int)(i - F);
+        } else if (r[u].i < total) {
+            const int b = (int)(r[u].i - F);
             const int c = __ldg(m.bnd_cell + b);
-            if (kind[b] == GF_BC_NONE) {
-                for (int k = 0; k < nc; ++k) out[k * total + i] = 0.0;
-                continue;
-            }
-            const double fr = frac[b];
-            const double vg = value_grad_coeff(m, b, fr);
-            for (int k = 0; k < nc; ++k)
-                out[k * total + i] = vg * (refv[k * nb + b] - psi[k * C + c]) + (1.0 - fr) * refg[k * nb + b];
+            const bool none = kind[b] == GF_BC_NONE;
+            const double fr = none ? 0.0 : frac[b];
+            const double vg = none ? 0.0 : value_grad_coeff(m, b, fr);
+#pragma unroll
+            for (int k = 0; k < NC; ++k)
+                out[k * total + r[u].i] =
+                    none ? 0.0 : vg * (refv[k * nb + b] - psi[k * C + c]) + (1.0 - fr) * refg[k * nb + b];
         }
     }
 }
@@ -1716,7 +1900,8 @@ int gf_bc_state(const gf_mesh_t* m, const gf_bc_t* bc, const double* psi, const 
     if (!valid_nc(bc->ncomp)) return GF_ERR_INVALID;
     if (m->n_bnd == 0) return GF_OK;
     gf_bc_aux_t a = aux ? *aux : gf_bc_aux_t{nullptr, nullptr, nullptr, nullptr, nullptr};
-    k_bc_state<<<grid_for(m->n_bnd), kThreads, 0, GF_STREAM(stream)>>>(*m, *bc, psi, a, *out);
+    auto kern = bc->ncomp == 1 ? k_bc_state<1> : k_bc_state<3>;
+    kern<<<grid_for(m->n_bnd, 128), 128, 0, GF_STREAM(stream)>>>(*m, *bc, psi, a, *out);
     return check_launch("gf_bc_state");
 }
 
@@ -1725,6 +1910,14 @@ int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8
     if (!valid_mesh(m) || !valid_nc(ncomp) || m->lsq_ata_inv == nullptr) return GF_ERR_INVALID;
     const unsigned g = grid_for(m->n_cells);
     cudaStream_t st = GF_STREAM(stream);
+    if (has_regular(m)) {
+        const double3 ih = make_double3(1.0 / m->reg_h[0], 1.0 / m->reg_h[1], 1.0 / m->reg_h[2]);
+        auto kern = m->stride_y > 0 ? (ncomp == 1 ? k_lsq_regular<1, true> : k_lsq_regular<3, true>)
+                                    : (ncomp == 1 ? k_lsq_regular<1, false> : k_lsq_regular<3, false>);
+        kern<<<g, kThreads, 0, st>>>(*m, ih, psi, grad);
+        lsq_list(m, ncomp, m->n_irr, m->irr_cells, psi, bc_kind, psib, grad, st);
+        return check_launch("gf_lsq_grad");
+    }
     const bool six = m->ell_width == 6 && m->n_faces < (int64_t)INT32_MAX;
     // Octree rows (6 < W <= 12, every row at least six slots): staged slots,
     // each row read to its last used slot.
@@ -1744,6 +1937,15 @@ int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8
             k_lsq_grad<3><<<g, kThreads, 0, st>>>(*m, psi, bc_kind, psib, grad);
     }
     return check_launch("gf_lsq_grad");
+}
+
+int gf_lsq_grad_hang(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8_t* bc_kind, const double* psib,
+                     double* grad, void* stream) {
+    if (!valid_mesh(m) || !valid_nc(ncomp) || m->lsq_ata_inv == nullptr) return GF_ERR_INVALID;
+    if (m->hang_cells == nullptr || m->ell_width < 6 || m->n_faces >= (int64_t)INT32_MAX)
+        return gf_lsq_grad(m, ncomp, psi, bc_kind, psib, grad, stream);
+    lsq_list(m, ncomp, m->n_hang_cells, m->hang_cells, psi, bc_kind, psib, grad, GF_STREAM(stream));
+    return check_launch("gf_lsq_grad_hang");
 }
 
 int gf_assemble(const gf_mesh_t* m, const gf_assembly_t* a, void* stream) {
@@ -1892,12 +2094,11 @@ int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel, const int8
         }
     }
     cudaStream_t st = GF_STREAM(stream);
-    if (m->face_axis != nullptr && grad_vel == nullptr && m->n_faces > 0 && m->n_faces < (int64_t)INT32_MAX) {
+    if (m->face_axis != nullptr && m->n_faces > 0 && m->n_faces < (int64_t)INT32_MAX) {
         const unsigned g = grid_for((m->n_faces + 1) / 2);
-        if (has)
-            k_face_flux_axis<true><<<g, kThreads, 0, st>>>(*m, vel, d, phi);
-        else
-            k_face_flux_axis<false><<<g, kThreads, 0, st>>>(*m, vel, d, phi);
+        auto kern = grad_vel != nullptr ? (has ? k_face_flux_axis<true, true> : k_face_flux_axis<false, true>)
+                                        : (has ? k_face_flux_axis<true, false> : k_face_flux_axis<false, false>);
+        kern<<<g, kThreads, 0, st>>>(*m, vel, d, grad_vel, phi);
         if (m->n_bnd > 0)
             k_face_flux<<<grid_for(m->n_bnd), kThreads, 0, st>>>(*m, mode, vel, u_kind, u_psib, d, has, grad_vel,
                                                                   phi, m->n_faces);
@@ -1940,16 +2141,18 @@ int gf_gauss_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi_f, double
 int gf_interpolate(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8_t* bc_kind, const double* psib,
                    const double* grad, double* out, void* stream) {
     if (!valid_mesh(m) || !valid_nc(ncomp)) return GF_ERR_INVALID;
-    k_interpolate<<<grid_for(m->n_faces + m->n_bnd), kThreads, 0, GF_STREAM(stream)>>>(*m, ncomp, psi, bc_kind,
-                                                                                       psib, grad, out);
+    const unsigned g = grid_for(m->n_faces + m->n_bnd, kThreads * kFaceRows);
+    auto kern = ncomp == 1 ? k_interpolate<1> : k_interpolate<3>;
+    kern<<<g, kThreads, 0, GF_STREAM(stream)>>>(*m, psi, bc_kind, psib, grad, out);
     return check_launch("gf_interpolate");
 }
 
 int gf_sn_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8_t* bc_kind, const double* frac,
                const double* refv, const double* refg, const double* grad, double* out, void* stream) {
     if (!valid_mesh(m) || !valid_nc(ncomp)) return GF_ERR_INVALID;
-    k_sn_grad<<<grid_for(m->n_faces + m->n_bnd), kThreads, 0, GF_STREAM(stream)>>>(*m, ncomp, psi, bc_kind, frac,
-                                                                                   refv, refg, grad, out);
+    const unsigned g = grid_for(m->n_faces + m->n_bnd, kThreads * kFaceRows);
+    auto kern = ncomp == 1 ? k_sn_grad<1> : k_sn_grad<3>;
+    kern<<<g, kThreads, 0, GF_STREAM(stream)>>>(*m, psi, bc_kind, frac, refv, refg, grad, out);
     return check_launch("gf_sn_grad");
 }
 

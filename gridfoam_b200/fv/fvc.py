@@ -61,21 +61,22 @@ def configured_grad(field: CellField, out: torch.Tensor, face_buf: torch.Tensor 
     g = None
     if grid.num_hanging > 0:
         g = lsq_buf if lsq_buf is not None else torch.empty((nc * 3, grid.num_cells), **f64)
-        call("gf_lsq_grad", ctypes.byref(grid.cmesh), nc, ptr(field.store), ptr(t.kind), ptr(t.psib), ptr(g), s)
+        call("gf_lsq_grad_hang", ctypes.byref(grid.cmesh), nc, ptr(field.store), ptr(t.kind), ptr(t.psib), ptr(g), s)
     call("gf_interpolate", ctypes.byref(grid.cmesh), nc, ptr(field.store), ptr(t.kind), ptr(t.psib), ptr(g),
          ptr(face_buf), s)
     call("gf_gauss_grad", ctypes.byref(grid.cmesh), nc, ptr(face_buf), ptr(out), s)
 
 
 def _hanging_grad(field: CellField) -> torch.Tensor | None:
-    """Least-squares gradient for the hanging-face corrections, or None on
-    meshes without hanging faces (boundary state must be current)."""
+    """Least-squares gradient for the hanging-face corrections (set at the
+    cells with a hanging face only), or None on meshes without hanging faces
+    (boundary state must be current)."""
     grid = field.grid
     if grid.num_hanging == 0:
         return None
     out = torch.empty((field.num_components * 3, grid.num_cells), dtype=torch.float64, device=grid.device)
     t = field.table
-    call("gf_lsq_grad", ctypes.byref(grid.cmesh), field.num_components, ptr(field.store), ptr(t.kind),
+    call("gf_lsq_grad_hang", ctypes.byref(grid.cmesh), field.num_components, ptr(field.store), ptr(t.kind),
          ptr(t.psib), ptr(out), stream_ptr())
     return out
 

@@ -43,26 +43,26 @@ def _base(field: CellField, mat: FvMatrix) -> GfAssembly:
     return a
 
 
-def _lsq_grad(field: CellField) -> torch.Tensor:
-    """Least-squares gradient (the hanging-face corrections always use it)."""
+def _lsq_grad(field: CellField, *, hanging_only: bool) -> torch.Tensor:
+    """Least-squares gradient; ``hanging_only``: set at the cells with a
+    hanging face only, all that the hanging-face corrections read."""
     grad = torch.empty((field.num_components * 3, field.grid.num_cells), dtype=torch.float64,
                        device=field.grid.device)
     t = field.table
-    call("gf_lsq_grad", ctypes.byref(field.grid.cmesh), field.num_components, ptr(field.store),
-         ptr(t.kind), ptr(t.psib), ptr(grad), stream_ptr())
+    call("gf_lsq_grad_hang" if hanging_only else "gf_lsq_grad", ctypes.byref(field.grid.cmesh), field.num_components,
+         ptr(field.store), ptr(t.kind), ptr(t.psib), ptr(grad), stream_ptr())
     return grad
 
 
-def _cfg_grad(field: CellField, lsq: torch.Tensor | None) -> torch.Tensor:
-    """The configured gradient (the TVD limiter's, schemes/div.py:302);
-    reuses ``lsq`` when the scheme is least squares."""
+def _cfg_grad(field: CellField) -> torch.Tensor:
+    """The configured gradient (the TVD limiter's, schemes/div.py:302)."""
     if schemes.grad_scheme(field.grid.sim_config, field.name) == GradScheme.LEASTSQUARE:
-        return lsq if lsq is not None else _lsq_grad(field)
+        return _lsq_grad(field, hanging_only=False)
     from gridfoam_b200.fv.fvc import configured_grad
 
     grad = torch.empty((field.num_components * 3, field.grid.num_cells), dtype=torch.float64,
                        device=field.grid.device)
-    configured_grad(field, grad, lsq_buf=lsq)
+    configured_grad(field, grad)
     return grad
 
 
@@ -144,11 +144,11 @@ def div(phi: FaceField, field: CellField) -> FvMatrix:
     if hanging and code == _lib.DIV_CODES["linear"]:
         # linear on hanging faces: the least-squares gradient of the offset
         # correction (schemes/div.py:134).
-        lsq = _lsq_grad(field)
+        lsq = _lsq_grad(field, hanging_only=True)
     if code >= _lib.DIV_CODES["vanleer"]:
         # TVD: the configured gradient, also in its hanging-face offset
         # correction (schemes/div.py:302).
-        grad = _cfg_grad(field, None)
+        grad = _cfg_grad(field)
     a = _base(field, mat)
     a.div_scheme = code
     a.div_sign = 1.0
@@ -188,7 +188,7 @@ def laplacian(gamma, field: CellField) -> FvMatrix:
     if grid.num_hanging > 0 and scheme in schemes.CORRECTED:
         # laplacian.py:162-176: explicit hanging-face skewness correction,
         # also kept as the matrix's face-flux correction.
-        grad = _lsq_grad(field)
+        grad = _lsq_grad(field, hanging_only=True)
         a.grad_lsq = ptr(grad)
         a.lap_corrected = 1
         mat._ffc = torch.zeros((field.num_components, grid.num_internal_faces), dtype=torch.float64,

@@ -121,6 +121,21 @@ typedef struct gf_mesh {
      * from ell_len[c] on hold boundary faces or nothing (zero matrix
      * coefficients), so row products may stop there. */
     const uint8_t* ell_len;
+    /* Regular cells, or NULL: reg_level[c] = L where cell c has exactly six
+     * faces, all internal and not immersed, to six neighbours of its own size
+     * reg_h * 2^L at that distance along the axes (255 elsewhere).  Their ELL
+     * slots are -x,+x,-y,+y,-z,+z and their geometry follows from L, so
+     * kernels read neither slot codes nor face or cell geometry for them.
+     * irr_cells lists the n_irr other cells. */
+    const uint8_t* reg_level;
+    const int32_t* irr_cells;
+    /* The n_hang_cells cells with a hanging face, or NULL. */
+    const int32_t* hang_cells;
+    int64_t n_irr;
+    int64_t n_hang_cells;
+    double reg_h[3];
+    /* > 0: uniform lexicographic box, neighbours c -+ 1, stride_y, stride_z */
+    int64_t stride_y, stride_z;
 } gf_mesh_t;
 
 /* Per-face boundary-condition table of one field (value-fraction form). */
@@ -254,6 +269,14 @@ int gf_bc_state(const gf_mesh_t* m, const gf_bc_t* bc, const double* psi,
 int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi,
                 const int8_t* bc_kind, const double* psib, double* grad,
                 void* stream);
+
+/* The same gradient at the cells with a hanging face only (mesh hang_cells;
+ * everywhere when that is NULL): all that the hanging-face corrections of
+ * interpolation, normal gradient, face flux, convection and Laplacian read.
+ * Other cells' values in grad are left as they are. */
+int gf_lsq_grad_hang(const gf_mesh_t* m, int32_t ncomp, const double* psi,
+                     const int8_t* bc_kind, const double* psib, double* grad,
+                     void* stream);
 
 /* fv/fvm/ddt.py:7-40, fv/fvm/div.py:15-73, fv/fvm/laplacian.py:101-201
  * (orthogonal part; meshes without hanging faces). */
