@@ -277,7 +277,8 @@ class GfError(RuntimeError):
 
 
 # Kernels launched per entry point (for launch accounting).
-_LAUNCHES_PER_CALL = {"gf_fixed_values": 3, "gf_close_fixed_flux": 2, "gf_field_residual": 2, "gf_continuity_sums": 2}
+_LAUNCHES_PER_CALL = {"gf_fixed_values": 3, "gf_close_fixed_flux": 2, "gf_field_residual": 2, "gf_continuity_sums": 2,
+                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2}
 LAUNCHES: collections.Counter = collections.Counter()
 # Launches known only after the device ran (the split CG's graph loop runs
 # two kernels an iteration): callables giving their counts, kept while

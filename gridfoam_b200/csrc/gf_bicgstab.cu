@@ -371,19 +371,6 @@ __global__ void __launch_bounds__(kT, 1) k_bicgstab(gf_krylov_t K) {
     bicgstab_body<NC, ROWS>(K, (int)blockIdx.x, (int)gridDim.x, sh, st);
 }
 
-template <int NC>
-__global__ void __launch_bounds__(kT, 1) k_bicgstab_batched(const KBatch B) {
-    __shared__ BiShared sh;
-    __shared__ BiState st[NC];
-    const int s = batch_system(B);
-    const gf_krylov_t& K = B.sys[s];
-    const int bid = (int)blockIdx.x - B.blk0[s], nb = B.blk0[s + 1] - B.blk0[s];
-    if (K.stride_y > 0)
-        bicgstab_body<NC, kBox>(K, bid, nb, sh, st);
-    else
-        bicgstab_body<NC, kEll>(K, bid, nb, sh, st);
-}
-
 }  // namespace
 
 template <int ROWS>
@@ -394,11 +381,6 @@ static const void* bi_kernel(int ncomp) {
 
 const void* bicgstab_kernel(const gf_krylov_t& k) {
     return k.stride_y > 0 ? bi_kernel<kBox>(k.ncomp) : (k.width == 6 ? bi_kernel<kEll6>(k.ncomp) : bi_kernel<kEll>(k.ncomp));
-}
-
-const void* bicgstab_batched_kernel(int ncomp) {
-    return ncomp == 1 ? (const void*)k_bicgstab_batched<1>
-                      : (ncomp == 2 ? (const void*)k_bicgstab_batched<2> : (const void*)k_bicgstab_batched<3>);
 }
 
 }  // namespace gf

@@ -52,12 +52,6 @@ static size_t cl_smem(int64_t chunk, int width) {
     return kClRedBytes + (size_t)chunk * (sizeof(double) + (size_t)width * (sizeof(double) + sizeof(uint32_t)));
 }
 
-template <int NSYS>
-struct ClBatch {
-    int chunk_of[NSYS];
-    gf_krylov_t sys[NSYS];
-};
-
 __device__ __forceinline__ unsigned cl_rank() {
     unsigned r;
     asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -239,15 +233,13 @@ __device__ __forceinline__ void cl_stats(double* o, double r0, double fin, int i
 // Jacobi-PCG with one reduction an iteration: w = A z and the sums |r|, r.z
 // and w.z, then the updates of p, q, x, r and z and one barrier that makes z
 // visible to the gathers.
-template <int WIDTH, int U, int NSYS>
-__global__ void __launch_bounds__(kClThreads, 1) k_cluster_cg(const __grid_constant__ ClBatch<NSYS> B) {
+template <int WIDTH, int U>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_cg(const __grid_constant__ gf_krylov_t K, int chunk) {
     extern __shared__ __align__(16) char cl_mem[];
     const unsigned rank = cl_rank(), size = cl_size();
-    const int sysi = NSYS == 1 ? 0 : (int)(blockIdx.x / size);
-    const gf_krylov_t& K = B.sys[sysi];
     ClReduce red(reinterpret_cast<double*>(cl_mem), size);
     ClRows<WIDTH, U> rows;
-    rows.init(K, cl_mem, B.chunk_of[sysi], rank);
+    rows.init(K, cl_mem, chunk, rank);
     const bool jac = K.jacobi != 0, linf = K.norm_inf != 0;
     double x[U], r[U], p[U], q[U], iv[U];
 #pragma unroll
@@ -325,17 +317,14 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_cg(const __grid_const
 // BiCGStab of one component: five cluster barriers an iteration (v; s; t;
 // r; the new direction).  The stopping tests, breakdown tests and restarts
 // are those of bicgstab_body, taken by every thread from the same sums.
-template <int WIDTH, int U, int NSYS>
-__global__ void __launch_bounds__(kClThreads, 1) k_cluster_bicgstab(const __grid_constant__ ClBatch<NSYS> B) {
+template <int WIDTH, int U>
+__global__ void __launch_bounds__(kClThreads, 1) k_cluster_bicgstab(const __grid_constant__ gf_krylov_t K, int chunk) {
     extern __shared__ __align__(16) char cl_mem[];
     const unsigned rank = cl_rank(), size = cl_size();
-    const int nc = B.sys[0].ncomp;
-    const int cl = (int)(blockIdx.x / size);
-    const int sysi = NSYS == 1 ? 0 : cl / nc, comp = NSYS == 1 ? cl : cl % nc;
-    const gf_krylov_t& K = B.sys[sysi];
+    const int comp = (int)(blockIdx.x / size);
     ClReduce red(reinterpret_cast<double*>(cl_mem), size);
     ClRows<WIDTH, U> rows;
-    rows.init(K, cl_mem, B.chunk_of[sysi], rank);
+    rows.init(K, cl_mem, chunk, rank);
     const bool jac = K.jacobi != 0, linf = K.norm_inf != 0;
     double* gx = K.x + (int64_t)comp * K.n;
     const double* rhs = K.rhs + (int64_t)comp * K.n;
@@ -535,7 +524,7 @@ static bool cluster_available() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 128) return false;
     std::lock_guard<std::mutex> lock(mu);
     if (known[dev] == 0) {
-        const void* kern = (const void*)k_cluster_cg<6, 11, 1>;
+        const void* kern = (const void*)k_cluster_cg<6, 11>;
         cudaLaunchAttribute at;
         at.id = cudaLaunchAttributeClusterDimension;
         at.val.clusterDim.x = kClBlocks;
@@ -570,72 +559,50 @@ bool cluster_fits(const gf_krylov_t& k, bool bicgstab) {
            cluster_available();
 }
 
-template <int WIDTH, int NSYS>
+template <int WIDTH>
 static const void* cl_kernel(int u, bool bicgstab) {
     if (bicgstab)
-        return u <= 1 ? (const void*)k_cluster_bicgstab<WIDTH, 1, NSYS>
-                      : (u <= 2 ? (const void*)k_cluster_bicgstab<WIDTH, 2, NSYS>
-                                : (u <= 4 ? (const void*)k_cluster_bicgstab<WIDTH, 4, NSYS>
-                                          : (const void*)k_cluster_bicgstab<WIDTH, 8, NSYS>));
-    return u <= 1 ? (const void*)k_cluster_cg<WIDTH, 1, NSYS>
-                  : (u <= 2 ? (const void*)k_cluster_cg<WIDTH, 2, NSYS>
-                            : (u <= 4 ? (const void*)k_cluster_cg<WIDTH, 4, NSYS>
-                                      : (u <= 8 ? (const void*)k_cluster_cg<WIDTH, 8, NSYS>
-                                                : (const void*)k_cluster_cg<WIDTH, 11, NSYS>)));
+        return u <= 1 ? (const void*)k_cluster_bicgstab<WIDTH, 1>
+                      : (u <= 2 ? (const void*)k_cluster_bicgstab<WIDTH, 2>
+                                : (u <= 4 ? (const void*)k_cluster_bicgstab<WIDTH, 4>
+                                          : (const void*)k_cluster_bicgstab<WIDTH, 8>));
+    return u <= 1 ? (const void*)k_cluster_cg<WIDTH, 1>
+                  : (u <= 2 ? (const void*)k_cluster_cg<WIDTH, 2>
+                            : (u <= 4 ? (const void*)k_cluster_cg<WIDTH, 4>
+                                      : (u <= 8 ? (const void*)k_cluster_cg<WIDTH, 8>
+                                                : (const void*)k_cluster_cg<WIDTH, 11>)));
 }
 
-template <int NSYS>
-static int launch_cluster_n(const gf_krylov_t* sys, int count, bool bicgstab, int fixed_size, cudaStream_t st) {
-    const char* what = bicgstab ? "gf_bicgstab_solve" : "gf_pcg_solve";
-    ClBatch<NSYS> B;
-    int64_t chunk = 0;
-    int width = 0;
-    bool six = true;
-    int size = 1;
+int launch_cluster(const gf_krylov_t* k, bool bicgstab, cudaStream_t st) {
     // One cell a thread as long as there are blocks: a cluster of one block
-    // up to 256 cells, then twice the blocks for twice the cells up to 16.  A
-    // batch always takes 16, so a system's sums do not depend on the others.
-    while (size < kClBlocks && (int64_t)size * kClThreads < sys[0].n) size *= 2;
-    if (fixed_size > 0) size = fixed_size;
-    for (int i = 0; i < count; ++i) {
-        if (!cluster_fits(sys[i], bicgstab)) return GF_ERR_INVALID;
-        B.sys[i] = sys[i];
-        const int64_t c = (sys[i].n + size - 1) / size;
-        B.chunk_of[i] = (int)c;
-        chunk = c > chunk ? c : chunk;
-        width = sys[i].width > width ? sys[i].width : width;
-        six = six && sys[i].width == 6;
-    }
-    const int threads = kClThreads;
-    const int u = (int)((chunk + threads - 1) / threads);
-    const void* kern = six ? cl_kernel<6, NSYS>(u, bicgstab) : cl_kernel<0, NSYS>(u, bicgstab);
-    const size_t smem = cl_smem(chunk, width);
+    // up to 256 cells, then twice the blocks for twice the cells up to 16.
+    int size = 1;
+    while (size < kClBlocks && (int64_t)size * kClThreads < k->n) size *= 2;
+    int chunk = (int)((k->n + size - 1) / size);
+    const int u = (chunk + kClThreads - 1) / kClThreads;
+    const void* kern = k->width == 6 ? cl_kernel<6>(u, bicgstab) : cl_kernel<0>(u, bicgstab);
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
     at.val.clusterDim.x = (unsigned)size;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(size * count * (bicgstab ? sys[0].ncomp : 1)));
-    cfg.blockDim = dim3((unsigned)threads);
-    cfg.dynamicSmemBytes = smem;
+    cfg.gridDim = dim3((unsigned)(size * (bicgstab ? k->ncomp : 1)));
+    cfg.blockDim = dim3((unsigned)kClThreads);
+    cfg.dynamicSmemBytes = cl_smem(chunk, k->width);
     cfg.stream = st;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    void* args[] = {&B};
+    gf_krylov_t arg = *k;
+    void* args[] = {&arg, &chunk};
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kClSmemMax);
     if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, kern, args);
     if (e != cudaSuccess) {
-        set_error("%s: cluster launch failed: %s", what, cudaGetErrorString(e));
+        set_error("%s: cluster launch failed: %s", bicgstab ? "gf_bicgstab_solve" : "gf_pcg_solve",
+                  cudaGetErrorString(e));
         return GF_ERR_CUDA;
     }
     return GF_OK;
-}
-
-int launch_cluster(const gf_krylov_t* sys, int count, bool bicgstab, bool batched, cudaStream_t st) {
-    if (count < 1 || count > kMaxBatch) return GF_ERR_INVALID;
-    return batched ? launch_cluster_n<kMaxBatch>(sys, count, bicgstab, kClBlocks, st)
-                   : launch_cluster_n<1>(sys, 1, bicgstab, 0, st);
 }
 
 }  // namespace gf

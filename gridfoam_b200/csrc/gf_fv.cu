@@ -478,8 +478,10 @@ __global__ void __launch_bounds__(kLsqThreads) k_lsq_list(gf_mesh_t m, int64_t n
     if (i < n) lsq_any_cell<NC>(m, __ldg(cells + i), psi, kind, psib, grad);
 }
 
-// Cells from which the regular cells get a kernel of their own.
-constexpr int64_t kRegularCells = 32768;
+// Cells from which the regular cells get a kernel of their own.  Below, a
+// gradient takes about 10 us either way, and the general kernel keeps the
+// bits that the distances between rounded cell centres give.
+constexpr int64_t kRegularCells = 131072;
 
 static bool has_regular(const gf_mesh_t* m) {
     return m->reg_level != nullptr && (m->irr_cells != nullptr || m->n_irr == 0) && m->n_cells >= kRegularCells &&

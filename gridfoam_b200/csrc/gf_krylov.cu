@@ -3339,6 +3339,337 @@ static BoxVariant sr_box_kernel(int variant) {
     }
 }
 
+// BiCGStab on a system's share of the blocks of a batched launch (a single
+// system goes to gf_bicgstab.cu or gf_cluster.cu).  A served case stops its
+// solves early (relative 0.1 and 0.01), and over its outer iterations the order
+// of a dot product's partial sums can show in the sixth digit, so this form
+// keeps its order of summation: a request gives the same bits as ever.
+//
+// WIDTH: the ELL row width at compile time (6) or 0 (any).  The Jacobi
+// inverse of every cell is computed once per solve into the workspace (after
+// the six vectors) and gathered from there by the preconditioned SpMVs.
+template <int NC, int WIDTH>
+__device__ void bicgstab_body(const gf_krylov_t& K, int vb, int vn) {
+    __shared__ BiState st[NC];
+    __shared__ int s_any;
+    KCtl* ctl = reinterpret_cast<KCtl*>(K.work);
+    const int bk = vb >= 0 ? vb : (int)blockIdx.x;
+    const int nbk = vn >= 0 ? vn : (int)gridDim.x;
+    barrier_init_v(K, nbk, bk);
+    double* partials = K.work + kCtlDoubles;
+    double* vec = partials + kPartials;
+    const int64_t n = K.n;
+    double* r = vec;
+    double* rh = vec + NC * n;
+    double* p = vec + 2 * NC * n;
+    double* v = vec + 3 * NC * n;
+    double* s = vec + 4 * NC * n;
+    double* t = vec + 5 * NC * n;
+    double* inv = vec + 6 * NC * n;
+    double* x = K.x;
+    const bool jac = K.jacobi != 0, linf = K.norm_inf != 0;
+    const int64_t t0 = bk * (int64_t)blockDim.x + threadIdx.x;
+    const int64_t stride = (int64_t)nbk * blockDim.x;
+    bool ok = true;
+
+    {  // r = b - A x; r_hat = p = r; |r|, r.r; the Jacobi inverse
+        double loc[2 * NC];
+#pragma unroll
+        for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
+        auto gx = [&](int k, int64_t i) { return __ldcg(x + k * n + i); };
+        for (int64_t c = t0; c < n; c += stride) {
+            __stcg(inv + c, inv_diag(K.diag, c, jac));
+            double ax[NC];
+            row_apply<NC, WIDTH>(K, c, gx, ax);
+#pragma unroll
+            for (int k = 0; k < NC; ++k) {
+                const double rk = __ldg(K.rhs + k * n + c) - ax[k];
+                __stcg(r + k * n + c, rk);
+                __stcg(rh + k * n + c, rk);
+                __stcg(p + k * n + c, rk);
+                loc[k] = norm_acc(loc[k], rk, linf);
+                loc[NC + k] += rk * rk;
+            }
+        }
+        ok = grid_reduce<2 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
+        if (threadIdx.x == 0) {
+            for (int k = 0; k < NC; ++k) {
+                BiState& b = st[k];
+                const double r0 = norm_fin(loc[k], linf);
+                b.r0 = r0;
+                b.final = r0;
+                b.thresh = fmax(K.atol, K.rtol * r0);
+                b.rho_old = loc[NC + k];
+                b.restarts = 0;
+                b.its = 0;
+                b.converged = 0;
+                b.status = GF_MAX_ITER;
+                b.mode = kRun;
+                if (r0 < b.thresh) {
+                    b.mode = kDone;
+                    b.converged = 1;
+                    b.status = GF_OK;
+                } else if (!isfinite(r0)) {
+                    b.mode = kDone;
+                    b.status = GF_NONFINITE;
+                }
+            }
+        }
+        __syncthreads();
+    }
+
+    for (int it = 1; ok && it <= K.max_iter; ++it) {
+        if (threadIdx.x == 0) {
+            int any = 0;
+            for (int k = 0; k < NC; ++k) {
+                if (st[k].mode == kIdle) st[k].mode = kRun;
+                any |= (st[k].mode == kRun);
+            }
+            s_any = any;
+        }
+        __syncthreads();
+        if (!s_any) break;
+
+        // P1: y = M p, v = A y; r_hat.v, |r_hat|^2, |v|^2
+        {
+            double loc[3 * NC];
+#pragma unroll
+            for (int j = 0; j < 3 * NC; ++j) loc[j] = 0.0;
+            auto gy = [&](int k, int64_t i) { return __ldcg(inv + i) * __ldcg(p + k * n + i); };
+            for (int64_t c = t0; c < n; c += stride) {
+                double av[NC];
+                row_apply<NC, WIDTH>(K, c, gy, av);
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    if (st[k].mode != kRun) continue;
+                    __stcg(v + k * n + c, av[k]);
+                    const double h = __ldcg(rh + k * n + c);
+                    loc[k] += h * av[k];
+                    loc[NC + k] += h * h;
+                    loc[2 * NC + k] += av[k] * av[k];
+                }
+            }
+            ok = grid_reduce<3 * NC>(ctl, partials, loc, 0u);
+            if (!ok) break;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < NC; ++k) {
+                    BiState& b = st[k];
+                    if (b.mode != kRun) continue;
+                    const double da = loc[k];
+                    if (fabs(da) <= 1e-6 * sqrt(loc[NC + k]) * sqrt(loc[2 * NC + k]))
+                        breakdown(b, it, K.max_restart);
+                    else
+                        b.alpha = b.rho_old / da;
+                }
+            }
+            __syncthreads();
+        }
+        // P2: s = r - alpha v, |s|; restarting systems copy r and reduce r.r
+        {
+            double loc[2 * NC];
+#pragma unroll
+            for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
+            for (int64_t c = t0; c < n; c += stride) {
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    const int md = st[k].mode;
+                    if (md == kRun) {
+                        const double sk = __ldcg(r + k * n + c) - st[k].alpha * __ldcg(v + k * n + c);
+                        __stcg(s + k * n + c, sk);
+                        loc[k] = norm_acc(loc[k], sk, linf);
+                    } else if (md == kRestart) {
+                        const double rk = __ldcg(r + k * n + c);
+                        __stcg(rh + k * n + c, rk);
+                        __stcg(p + k * n + c, rk);
+                        loc[NC + k] += rk * rk;
+                    }
+                }
+            }
+            ok = grid_reduce<2 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
+            if (!ok) break;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < NC; ++k) {
+                    BiState& b = st[k];
+                    if (b.mode == kRestart) {
+                        b.rho_old = loc[NC + k];
+                        b.mode = kIdle;
+                    } else if (b.mode == kRun) {
+                        const double fin = norm_fin(loc[k], linf);
+                        b.final = fin;
+                        if (fin < b.thresh) {
+                            b.mode = kConvS;
+                            b.converged = 1;
+                            b.its = it;
+                            b.status = GF_OK;
+                        } else if (!isfinite(fin)) {
+                            b.mode = kDone;
+                            b.its = it;
+                            b.status = GF_NONFINITE;
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        // P3: converged-on-s systems take x += alpha y; others z = M s, t = A z
+        {
+            double loc[2 * NC];
+#pragma unroll
+            for (int j = 0; j < 2 * NC; ++j) loc[j] = 0.0;
+            auto gz = [&](int k, int64_t i) { return __ldcg(inv + i) * __ldcg(s + k * n + i); };
+            for (int64_t c = t0; c < n; c += stride) {
+                double at[NC];
+                row_apply<NC, WIDTH>(K, c, gz, at);
+                const double ic = __ldcg(inv + c);
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    const int md = st[k].mode;
+                    if (md == kConvS) {
+                        const double y = ic * __ldcg(p + k * n + c);
+                        __stcg(x + k * n + c, __ldcg(x + k * n + c) + st[k].alpha * y);
+                    } else if (md == kRun) {
+                        __stcg(t + k * n + c, at[k]);
+                        loc[k] += at[k] * at[k];
+                        loc[NC + k] += at[k] * __ldcg(s + k * n + c);
+                    }
+                }
+            }
+            ok = grid_reduce<2 * NC>(ctl, partials, loc, 0u);
+            if (!ok) break;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < NC; ++k) {
+                    BiState& b = st[k];
+                    if (b.mode == kConvS) {
+                        b.mode = kDone;
+                        continue;
+                    }
+                    if (b.mode != kRun) continue;
+                    const double dd = loc[k];
+                    const double tn = sqrt(loc[k]);
+                    if (fabs(dd) <= 1e-6 * tn * tn) {
+                        breakdown(b, it, K.max_restart);
+                        continue;
+                    }
+                    b.omega = loc[NC + k] / dd;
+                    if (fabs(b.omega) <= 1e-6) breakdown(b, it, K.max_restart);
+                }
+            }
+            __syncthreads();
+        }
+        // P4: x += alpha y + omega z, r = s - omega t; |r|, r_hat.r, |r_hat|^2, |r|^2
+        {
+            double loc[4 * NC];
+#pragma unroll
+            for (int j = 0; j < 4 * NC; ++j) loc[j] = 0.0;
+            for (int64_t c = t0; c < n; c += stride) {
+                const double ic = __ldcg(inv + c);
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    const int md = st[k].mode;
+                    if (md == kRun) {
+                        const double sk = __ldcg(s + k * n + c);
+                        const double y = ic * __ldcg(p + k * n + c);
+                        const double z = ic * sk;
+                        __stcg(x + k * n + c, __ldcg(x + k * n + c) + st[k].alpha * y + st[k].omega * z);
+                        const double rk = sk - st[k].omega * __ldcg(t + k * n + c);
+                        __stcg(r + k * n + c, rk);
+                        const double h = __ldcg(rh + k * n + c);
+                        loc[k] = norm_acc(loc[k], rk, linf);
+                        loc[NC + k] += h * rk;
+                        loc[2 * NC + k] += h * h;
+                        loc[3 * NC + k] += rk * rk;
+                    } else if (md == kRestart) {
+                        const double rk = __ldcg(r + k * n + c);
+                        __stcg(rh + k * n + c, rk);
+                        __stcg(p + k * n + c, rk);
+                        loc[3 * NC + k] += rk * rk;
+                    }
+                }
+            }
+            ok = grid_reduce<4 * NC>(ctl, partials, loc, linf ? ((1u << NC) - 1u) : 0u);
+            if (!ok) break;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < NC; ++k) {
+                    BiState& b = st[k];
+                    if (b.mode == kRestart) {
+                        b.rho_old = loc[3 * NC + k];
+                        b.mode = kIdle;
+                        continue;
+                    }
+                    if (b.mode != kRun) continue;
+                    const double fin = norm_fin(loc[k], linf);
+                    b.final = fin;
+                    if (fin < b.thresh) {
+                        b.mode = kDone;
+                        b.converged = 1;
+                        b.its = it;
+                        b.status = GF_OK;
+                        continue;
+                    }
+                    if (!isfinite(fin)) {
+                        b.mode = kDone;
+                        b.its = it;
+                        b.status = GF_NONFINITE;
+                        continue;
+                    }
+                    const double rho_new = loc[NC + k];
+                    if (fabs(rho_new) <= 1e-6 * sqrt(loc[2 * NC + k]) * sqrt(loc[3 * NC + k])) {
+                        breakdown(b, it, K.max_restart);
+                        continue;
+                    }
+                    b.beta = (rho_new / b.rho_old) * (b.alpha / b.omega);
+                    b.rho_old = rho_new;
+                }
+            }
+            __syncthreads();
+        }
+        // P5: p = r + beta (p - omega v); restarting systems copy r
+        {
+            double loc[NC];
+#pragma unroll
+            for (int k = 0; k < NC; ++k) loc[k] = 0.0;
+            for (int64_t c = t0; c < n; c += stride) {
+#pragma unroll
+                for (int k = 0; k < NC; ++k) {
+                    const int md = st[k].mode;
+                    if (md == kRun) {
+                        const double pk = __ldcg(p + k * n + c);
+                        __stcg(p + k * n + c,
+                               __ldcg(r + k * n + c) + st[k].beta * (pk - st[k].omega * __ldcg(v + k * n + c)));
+                    } else if (md == kRestart) {
+                        const double rk = __ldcg(r + k * n + c);
+                        __stcg(rh + k * n + c, rk);
+                        __stcg(p + k * n + c, rk);
+                        loc[k] += rk * rk;
+                    }
+                }
+            }
+            ok = grid_reduce<NC>(ctl, partials, loc, 0u);
+            if (!ok) break;
+            if (threadIdx.x == 0) {
+                for (int k = 0; k < NC; ++k) {
+                    if (st[k].mode == kRestart) {
+                        st[k].rho_old = loc[k];
+                        st[k].mode = kIdle;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    if (bk == 0 && threadIdx.x == 0) {
+        for (int k = 0; k < NC; ++k) {
+            double* o = K.stats + 5 * k;
+            const bool fin = st[k].mode == kDone;
+            o[0] = st[k].r0;
+            o[1] = st[k].final;
+            o[2] = fin ? st[k].its : K.max_iter;
+            o[3] = st[k].converged;
+            o[4] = ok ? (fin ? st[k].status : GF_MAX_ITER) : GF_ERR_TIMEOUT;
+        }
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Mixed precision BiCGStab: FP32 inner BiCGStab cycles inside FP64
 // iterative refinement, for all NC components in one launch.  Each cycle
@@ -4368,6 +4699,20 @@ static int launch_split(const gf_krylov_t* k, void* stream, int which) {
 // blocks [blk0[i], blk0[i+1]) and runs the single-system kernel's body on
 // them with its own barrier counter and partials (its workspace), so its
 // iterates do not depend on which other systems share the launch.
+constexpr int kMaxBatch = 16;
+
+struct KBatch {
+    int count;
+    int blk0[kMaxBatch + 1];
+    gf_krylov_t sys[kMaxBatch];
+};
+
+__device__ __forceinline__ int batch_system(const KBatch& B) {
+    int s = 0;
+    while (s + 1 < B.count && (int)blockIdx.x >= B.blk0[s + 1]) ++s;
+    return s;
+}
+
 // Zeroes every system's barrier control block (one launch for the batch).
 __global__ void k_batch_reset(const KBatch B) {
     for (int i = threadIdx.x; i < B.count; i += blockDim.x) {
@@ -4416,6 +4761,17 @@ __global__ void __launch_bounds__(kCgThreads, 4) k_pcg1_batched(const KBatch B) 
         EllRows<double, 0> rows{K.val, K.nbr, K.n, K.width, K.row_len};
         pcg1_body<kCgThreads, 1>(K, rows, bid, nb);
     }
+}
+
+template <int NC>
+__global__ void __launch_bounds__(kKThreads) k_bicgstab_batched(const KBatch B) {
+    const int s = batch_system(B);
+    const gf_krylov_t& K = B.sys[s];
+    const int bid = (int)blockIdx.x - B.blk0[s], nb = B.blk0[s + 1] - B.blk0[s];
+    if (K.width == 6)
+        bicgstab_body<NC, 6>(K, bid, nb);
+    else
+        bicgstab_body<NC, 0>(K, bid, nb);
 }
 
 template <class Kern>
@@ -4830,7 +5186,7 @@ int gf_pcg_solve(const gf_krylov_t* k, void* stream) {
                 if (st != GF_ERR_INVALID) return st;
             }
             if (k->variant == kHaloVariant && cluster_fits(*k, false))
-                return launch_cluster(k, 1, false, false, reinterpret_cast<cudaStream_t>(stream));
+                return launch_cluster(k, false, reinterpret_cast<cudaStream_t>(stream));
             if (k->variant == kHaloVariant) {
                 int st = launch_resident(k, reinterpret_cast<cudaStream_t>(stream));
                 if (st != GF_ERR_INVALID) return st;
@@ -4911,7 +5267,7 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream) {
         set_error("gf_bicgstab_solve: a box layout needs width 6 and strides 1 <= stride_y <= stride_z");
         return GF_ERR_INVALID;
     }
-    if (cluster_fits(*k, true)) return launch_cluster(k, 1, true, false, reinterpret_cast<cudaStream_t>(stream));
+    if (cluster_fits(*k, true)) return launch_cluster(k, true, reinterpret_cast<cudaStream_t>(stream));
     return launch_persistent(bicgstab_kernel(*k), k, stream, "gf_bicgstab_solve", kBicgThreads);
 }
 
@@ -4928,8 +5284,8 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
     }
     KBatch B;
     memset(&B, 0, sizeof(B));
-    gf_krylov_t small[kMaxBatch];
-    int nsmall = 0, total = 0, nblk = 0;
+    B.count = count;
+    int total = 0;
     for (int i = 0; i < count; ++i) {
         const gf_krylov_t& k = sys[i];
         if (k.mixed && bicg) {
@@ -4961,21 +5317,16 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
             set_error("%s: system %d: block count %d outside 1..%d", what, i, blocks[i], kMaxBlocks);
             return GF_ERR_INVALID;
         }
+        B.sys[i] = k;
+        B.blk0[i] = total;
         total += blocks[i];
-        // A system's route depends on itself alone, so its bits do not
-        // depend on the others: one cluster where it fits, else its share of
-        // the cooperative launch.
-        if (cluster_fits(k, bicg)) {
-            small[nsmall++] = k;
-            continue;
-        }
-        B.sys[B.count] = k;
-        B.blk0[B.count++] = nblk;
-        nblk += blocks[i];
     }
-    B.blk0[B.count] = nblk;
-    const void* kern = bicg ? bicgstab_batched_kernel(sys[0].ncomp) : (const void*)k_pcg1_batched;
-    const int threads = bicg ? kBicgThreads : kCgThreads;
+    B.blk0[count] = total;
+    const void* kern = !bicg ? (const void*)k_pcg1_batched
+                             : (sys[0].ncomp == 1 ? (const void*)k_bicgstab_batched<1>
+                                                  : sys[0].ncomp == 2 ? (const void*)k_bicgstab_batched<2>
+                                                                      : (const void*)k_bicgstab_batched<3>);
+    const int threads = bicg ? kKThreads : kCgThreads;
     int dev = 0, sms = 0, coop = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -4990,10 +5341,6 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
         return GF_ERR_INVALID;
     }
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
-    if (nsmall > 0) {
-        const int rc = launch_cluster(small, nsmall, bicg, true, st);
-        if (rc != GF_OK || B.count == 0) return rc;
-    }
     k_batch_reset<<<1, 32, 0, st>>>(B);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -5001,7 +5348,7 @@ static int launch_batched(const gf_krylov_t* sys, int32_t count, const int32_t* 
         return GF_ERR_CUDA;
     }
     void* args[] = {&B};
-    e = cudaLaunchCooperativeKernel(kern, dim3(nblk), dim3(threads), args, 0, st);
+    e = cudaLaunchCooperativeKernel(kern, dim3(total), dim3(threads), args, 0, st);
     if (e != cudaSuccess) {
         set_error("%s: cooperative launch failed: %s", what, cudaGetErrorString(e));
         return GF_ERR_CUDA;
@@ -5020,10 +5367,10 @@ int gf_bicgstab_solve_batched(const gf_krylov_t* systems, int32_t count, const i
 }
 
 int gf_batch_max_blocks(int32_t bicgstab) {
-    const void* kern = bicgstab ? bicgstab_batched_kernel(3) : (const void*)k_pcg1_batched;
+    const void* kern = bicgstab ? (const void*)k_bicgstab_batched<3> : (const void*)k_pcg1_batched;
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
-        cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bicgstab ? kBicgThreads : kCgThreads,
+        cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bicgstab ? kKThreads : kCgThreads,
                                                                       0) != cudaSuccess) {
         set_error("gf_batch_max_blocks: device query failed");
         return -1;

@@ -6,7 +6,6 @@
 
 namespace gf {
 
-constexpr int kMaxBatch = 16;  // systems of a batched launch
 constexpr int kMaxBlocks = 1024;
 constexpr int kMaxNV = 16;
 constexpr int kCtlDoubles = 32;
@@ -77,23 +76,8 @@ __device__ __forceinline__ void breakdown(BiState& s, int it, int max_restart) {
     }
 }
 
-// The systems of a batched cooperative launch: system i owns the blocks
-// [blk0[i], blk0[i+1]).
-struct KBatch {
-    int count;
-    int blk0[kMaxBatch + 1];
-    gf_krylov_t sys[kMaxBatch];
-};
-
-__device__ __forceinline__ int batch_system(const KBatch& B) {
-    int s = 0;
-    while (s + 1 < B.count && (int)blockIdx.x >= B.blk0[s + 1]) ++s;
-    return s;
-}
-
 // Grid BiCGStab kernels (gf_bicgstab.cu).
 const void* bicgstab_kernel(const gf_krylov_t& k);
-const void* bicgstab_batched_kernel(int ncomp);
 constexpr int kBicgThreads = 1024;
 
 // Halo flags: one 64-bit epoch per block, one per 128-byte line (flags of
@@ -106,10 +90,9 @@ constexpr int64_t kHaloFlagDoubles = kMaxBlocks * kHaloFlagStride;
 // GF_ERR_INVALID without a launch when it does not fit.
 int launch_resident(const gf_krylov_t* k, cudaStream_t st);
 
-// Solves on one thread-block cluster a system (gf_cluster.cu).  The launch
-// functions return GF_ERR_INVALID without a launch when a system does not
-// qualify; cluster_fits says so beforehand.
+// A solve on one thread-block cluster (gf_cluster.cu), for a system that
+// cluster_fits.
 bool cluster_fits(const gf_krylov_t& k, bool bicgstab);
-int launch_cluster(const gf_krylov_t* sys, int count, bool bicgstab, bool batched, cudaStream_t st);
+int launch_cluster(const gf_krylov_t* k, bool bicgstab, cudaStream_t st);
 
 }  // namespace gf

@@ -23,14 +23,14 @@ def _grid(name):
     from gridfoam_b200.meta.config import SimulatorConfig
 
     if name == "wake":
-        case = cylinder_wake_case((52, 38, 8))
+        case = cylinder_wake_case((80, 54, 10))
     else:
         case = pipe_case(33, 34)
-        case["mesh"] |= {"res": [33, 35, 37], "upper": [33 / 64, 35 / 64, 37 / 64]}
-        case["mesh"]["bodies"] = [case["mesh"]["bodies"][0] | {"center": [0.26, 0.27], "radius": 0.2}] * (name == "pipe")
+        case["mesh"] |= {"res": [51, 53, 55], "upper": [51 / 64, 53 / 64, 55 / 64]}
+        case["mesh"]["bodies"] = [case["mesh"]["bodies"][0] | {"center": [0.4, 0.41], "radius": 0.3}] * (name == "pipe")
     grid = AxisProjectedGrid(SimulatorConfig.model_validate(case["simulator"]), build_mesh(case["mesh"], device="cuda"),
                              device="cuda")
-    assert grid.num_cells >= 32768  # the size from which the regular cells get their own path
+    assert grid.num_cells >= 131072  # the size from which the regular cells get their own path
     return grid
 
 
