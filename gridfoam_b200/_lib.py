@@ -224,6 +224,7 @@ _SIGNATURES = {
     "gf_adjust_phi": ([P, P, P, P], ctypes.c_int),
     "gf_relax_field": ([I64, F64, P, P, P], ctypes.c_int),
     "gf_axpby": ([I64, F64, P, F64, P, P, P], ctypes.c_int),
+    "gf_matrix_axpby": ([P, I32, F64, P, P, P, F64, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_ell_to_ldu": ([P, P, P, P, P], ctypes.c_int),
     "gf_ldu_to_ell": ([P, P, P, P, P], ctypes.c_int),
     "gf_field_residual": ([P, I32, P, P, P, P, P, P, P], ctypes.c_int),

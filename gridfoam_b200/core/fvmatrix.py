@@ -44,15 +44,18 @@ def fixed_values_ldu(grid, diag: torch.Tensor, upper: torch.Tensor, lower: torch
 
 
 class FvMatrix:
-    def __init__(self, field: CellField, *, _alloc: bool = True):
+    def __init__(self, field: CellField, *, _alloc: bool = True, _zero: bool = True):
+        """``_zero=False``: the arrays are left unset, for an operator that
+        writes every entry."""
         self._field = field
         self._grid = field.grid
         g = self._grid
         nc = field.num_components
         if _alloc:
-            self.diag_store = torch.zeros(g.num_cells, dtype=torch.float64, device=g.device)
-            self.val = torch.zeros(g.ell_width * g.num_cells, dtype=torch.float64, device=g.device)
-            self.source_store = torch.zeros((nc, g.num_cells), dtype=torch.float64, device=g.device)
+            new = torch.zeros if _zero else torch.empty
+            self.diag_store = new(g.num_cells, dtype=torch.float64, device=g.device)
+            self.val = new(g.ell_width * g.num_cells, dtype=torch.float64, device=g.device)
+            self.source_store = new((nc, g.num_cells), dtype=torch.float64, device=g.device)
         # Explicit face-flux correction [nc][F] on internal faces (zero off
         # hanging faces), or None: FvMatrix.face_flux_correction.
         self._ffc: torch.Tensor | None = None
@@ -194,14 +197,11 @@ class FvMatrix:
 
     # ------------------------------------------------------------------
     def _combine(self, other: "FvMatrix", a: float, b: float) -> "FvMatrix":
-        res = FvMatrix(self._field)
-        s = stream_ptr()
-        for x, y, out in (
-            (self.diag_store, other.diag_store, res.diag_store),
-            (self.val, other.val, res.val),
-            (self.source_store, other.source_store, res.source_store),
-        ):
-            call("gf_axpby", x.numel(), a, ptr(x), b, ptr(y), ptr(out), s)
+        res = FvMatrix(self._field, _zero=False)
+        call("gf_matrix_axpby", ctypes_ref(self._grid.cmesh), self.num_components,
+             a, ptr(self.diag_store), ptr(self.val), ptr(self.source_store),
+             b, ptr(other.diag_store), ptr(other.val), ptr(other.source_store),
+             ptr(res.diag_store), ptr(res.val), ptr(res.source_store), stream_ptr())
         res._ffc = self._combine_ffc(self._ffc, other._ffc, a, b)
         if self.requires_grad or other.requires_grad:
             xs, ys = self.autograd_tensors(), other.autograd_tensors()

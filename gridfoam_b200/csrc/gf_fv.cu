@@ -721,6 +721,8 @@ __global__ void __launch_bounds__(256, 2) k_assemble6(gf_mesh_t m, gf_assembly_t
     for (int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; c < C;
          c += (int64_t)gridDim.x * blockDim.x) {
         int code[W], nbr[W], fc[W], imm[W];
+        const bool look = m.n_imm > 0 && m.imm_index != nullptr &&
+                          (m.reg_level == nullptr || __ldg(m.reg_level + c) == 255);
 #pragma unroll
         for (int s = 0; s < W; ++s) {
             code[s] = __ldg(m.ell_code + s * C + c);
@@ -730,7 +732,7 @@ __global__ void __launch_bounds__(256, 2) k_assemble6(gf_mesh_t m, gf_assembly_t
         for (int s = 0; s < W; ++s) {
             const int f = code[s] >> 1;
             fc[s] = (code[s] >= 0 && f < F) ? f : 0;
-            imm[s] = m.imm_index ? __ldg(m.imm_index + fc[s]) : -1;
+            imm[s] = look ? __ldg(m.imm_index + fc[s]) : -1;
         }
         double w[W], phi[W], msf[W], dl[W], go[W], gn[W];
 #pragma unroll
@@ -860,6 +862,8 @@ __device__ __forceinline__ void assemble_slots(const gf_mesh_t& m, const gf_asse
     const int F = (int)m.n_faces;
     const int64_t nb = m.n_bnd;
     const bool linear = a.div_scheme == GF_DIV_LINEAR;
+    // a regular cell (mesh reg_level) has no immersed and no hanging face
+    const bool look = m.reg_level == nullptr || __ldg(m.reg_level + c) == 255;
     int code[G], nbr[G], fc[G], imm[G], hg[G];
 #pragma unroll
     for (int s = 0; s < G; ++s) {
@@ -871,8 +875,8 @@ __device__ __forceinline__ void assemble_slots(const gf_mesh_t& m, const gf_asse
     for (int s = 0; s < G; ++s) {
         const int f = code[s] >> 1;
         fc[s] = (code[s] >= 0 && f < F) ? f : 0;
-        imm[s] = m.imm_index ? __ldg(m.imm_index + fc[s]) : -1;
-        hg[s] = hang_of(m, fc[s]);
+        imm[s] = look && m.n_imm > 0 && m.imm_index ? __ldg(m.imm_index + fc[s]) : -1;
+        hg[s] = look ? hang_of(m, fc[s]) : -1;
     }
     double w[G], phi[G], msf[G], dl[G], go[G], gn[G];
 #pragma unroll
@@ -1035,6 +1039,61 @@ __global__ void __launch_bounds__(256, 2) k_assemble12(gf_mesh_t m, gf_assembly_
 #pragma unroll
         for (int k = 0; k < NC; ++k) a.source[k * C + c] = src[k];
     }
+}
+
+// The time derivative alone (no convection, no Laplacian): a diagonal, a
+// source and zero couplings.  No slot is read (through the Laplacian form with
+// its sign zero it cost as much as that, 436 us on a 4.08M-cell octree).
+template <int NC>
+__global__ void __launch_bounds__(256) k_assemble_ddt(gf_mesh_t m, gf_assembly_t a) {
+    const int64_t C = m.n_cells;
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= C) return;
+    const double vdt = a.use_ddt ? __ldg(m.volume + c) / a.dt : 0.0;
+    double hist[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) {
+        hist[k] = a.use_ddt ? a.ddt_b * a.psi_old[k * C + c] : 0.0;
+        if (a.use_ddt && a.ddt_c != 0.0) hist[k] = hist[k] - a.ddt_c * a.psi_older[k * C + c];
+    }
+    for (int s = 0; s < m.ell_width; ++s) a.val[s * C + c] = 0.0;
+    a.diag[c] = a.ddt_a * vdt;
+#pragma unroll
+    for (int k = 0; k < NC; ++k) a.source[k * C + c] = vdt * hist[k];
+}
+
+// out = a x + b y of two matrices: diagonal, couplings and source in one pass.
+// Slots past a row's last coupling (ell_len) are zero in both and only
+// written: of twelve slots a row of an octree six are padding as a rule.
+template <int NC>
+__global__ void __launch_bounds__(256) k_matrix_axpby(gf_mesh_t m, double a, const double* __restrict__ xd,
+                                                      const double* __restrict__ xv, const double* __restrict__ xs,
+                                                      double b, const double* __restrict__ yd,
+                                                      const double* __restrict__ yv, const double* __restrict__ ys,
+                                                      double* __restrict__ od, double* __restrict__ ov,
+                                                      double* __restrict__ os) {
+    const int64_t C = m.n_cells;
+    const int64_t c = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (c >= C) return;
+    const int W = m.ell_width, len = m.ell_len ? (int)__ldg(m.ell_len + c) : W;
+    const double d = a * xd[c] + b * yd[c];
+    double src[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) src[k] = a * xs[k * C + c] + b * ys[k * C + c];
+    for (int s0 = 0; s0 < W; s0 += 6) {
+        double x[6], y[6];
+#pragma unroll
+        for (int s = 0; s < 6; ++s) {
+            x[s] = s0 + s < len ? xv[(s0 + s) * C + c] : 0.0;
+            y[s] = s0 + s < len ? yv[(s0 + s) * C + c] : 0.0;
+        }
+#pragma unroll
+        for (int s = 0; s < 6; ++s)
+            if (s0 + s < W) ov[(s0 + s) * C + c] = s0 + s < len ? a * x[s] + b * y[s] : 0.0;
+    }
+    od[c] = d;
+#pragma unroll
+    for (int k = 0; k < NC; ++k) os[k * C + c] = src[k];
 }
 
 __global__ void k_momentum_finalize(int64_t C, int nc, double relax, const double* __restrict__ vol,
@@ -1977,7 +2036,10 @@ int gf_assemble(const gf_mesh_t* m, const gf_assembly_t* a, void* stream) {
     const bool conv = a->div_scheme != GF_DIV_NONE, lap = a->lap_sign != 0.0;
     cudaStream_t st = GF_STREAM(stream);
     const unsigned g = grid_for(m->n_cells);
-    if (fast) {
+    if (!conv && !lap && a->ffc == nullptr) {
+        if (a->ncomp == 1) k_assemble_ddt<1><<<g, kThreads, 0, st>>>(*m, *a);
+        else k_assemble_ddt<3><<<g, kThreads, 0, st>>>(*m, *a);
+    } else if (fast) {
         if (a->ncomp == 1) {
             if (conv && lap) k_assemble6<1, true, true><<<g, kThreads, 0, st>>>(*m, *a);
             else if (conv) k_assemble6<1, true, false><<<g, kThreads, 0, st>>>(*m, *a);
@@ -2218,6 +2280,21 @@ int gf_axpby(int64_t n, double a, const double* x, double b, const double* y, do
     if (n == 0) return GF_OK;
     k_axpby<<<grid_for(n), kThreads, 0, GF_STREAM(stream)>>>(n, a, x, b, y, out);
     return check_launch("gf_axpby");
+}
+
+int gf_matrix_axpby(const gf_mesh_t* m, int32_t ncomp, double a, const double* xdiag, const double* xval,
+                    const double* xsource, double b, const double* ydiag, const double* yval, const double* ysource,
+                    double* diag, double* val, double* source, void* stream) {
+    if (!valid_mesh(m) || !valid_nc(ncomp)) return GF_ERR_INVALID;
+    if (xdiag == nullptr || xval == nullptr || xsource == nullptr || ydiag == nullptr || yval == nullptr ||
+        ysource == nullptr || diag == nullptr || val == nullptr || source == nullptr) {
+        set_error("gf_matrix_axpby: null array");
+        return GF_ERR_INVALID;
+    }
+    auto kern = ncomp == 1 ? k_matrix_axpby<1> : k_matrix_axpby<3>;
+    kern<<<grid_for(m->n_cells), kThreads, 0, GF_STREAM(stream)>>>(*m, a, xdiag, xval, xsource, b, ydiag, yval,
+                                                                   ysource, diag, val, source);
+    return check_launch("gf_matrix_axpby");
 }
 
 int gf_ell_to_ldu(const gf_mesh_t* m, const double* val, double* upper, double* lower, void* stream) {

@@ -119,7 +119,7 @@ def _attach(mat: FvMatrix, param: torch.Tensor, kernel: str, a: GfAssembly, keep
 
 def ddt(field: CellField) -> FvMatrix:
     """fv/fvm/ddt.py:7-40."""
-    mat = FvMatrix(field)
+    mat = FvMatrix(field, _zero=False)
     _eval_state(field)
     a = _base(field, mat)
     ca, cb, cc = schemes.ddt_coefficients(field)
@@ -135,7 +135,7 @@ def div(phi: FaceField, field: CellField) -> FvMatrix:
     """fv/fvm/div.py:15-73 with the configured scheme."""
     if phi.component_shape != ():
         raise ValueError("convection requires scalar face flux")
-    mat = FvMatrix(field)
+    mat = FvMatrix(field, _zero=False)
     _eval_state(field)
     scheme = schemes.div_scheme(field.grid.sim_config, phi.name, field.name)
     code = _lib.DIV_CODES[scheme.value]
@@ -168,7 +168,7 @@ def div(phi: FaceField, field: CellField) -> FvMatrix:
 def laplacian(gamma, field: CellField) -> FvMatrix:
     """fv/fvm/laplacian.py:101-201 (uniform or per-cell diffusivity)."""
     grid = field.grid
-    mat = FvMatrix(field)
+    mat = FvMatrix(field, _zero=False)
     _eval_state(field)
     scheme = schemes.laplacian_scheme(grid.sim_config, field.name)
     a = _base(field, mat)

@@ -470,6 +470,14 @@ int gf_relax_field(int64_t n, double alpha, const double* old, double* cur,
 int gf_axpby(int64_t n, double a, const double* x, double b, const double* y,
              double* out, void* stream);
 
+/* out = a x + b y of two matrices (diag [C], val [W][C], source [ncomp][C]);
+ * slots past ell_len are taken as zero and written so. */
+int gf_matrix_axpby(const gf_mesh_t* m, int32_t ncomp, double a,
+                    const double* xdiag, const double* xval,
+                    const double* xsource, double b, const double* ydiag,
+                    const double* yval, const double* ysource, double* diag,
+                    double* val, double* source, void* stream);
+
 /* LDU <-> ELL conversions for the FvMatrix.upper/lower API. */
 int gf_ell_to_ldu(const gf_mesh_t* m, const double* val, double* upper,
                   double* lower, void* stream);
