@@ -4170,21 +4170,19 @@ __device__ __forceinline__ SplitVec split_vec(const gf_krylov_t& K) {
     return {vec, vec + n, vec + 2 * n, vec + 3 * n, vec + 4 * n, partials, partials + kMaxBlocks};
 }
 
-// L2 prefetch of one address (a hint: no register result, no fault; every
-// address given is inside its array).
-__device__ __forceinline__ void pf_l2(const void* p) { asm volatile("prefetch.L2 [%0];" ::"l"(p)); }
-
-// The first slots (up to six) of row c of an ELL operator: what the row
-// kernel's first pass reads of the matrix.  Box operators: nothing.
-template <class Rows>
-__device__ __forceinline__ void split_prefetch_rows(const Rows&, int) {}
-template <typename T, int WIDTH, typename I, int GRP>
-__device__ __forceinline__ void split_prefetch_rows(const EllRows<T, WIDTH, I, GRP>& r, int c) {
-    const int ws = WIDTH > 0 ? WIDTH : (r.w < 6 ? r.w : 6);
-    for (int s = 0; s < ws; ++s) {
-        pf_l2(r.val + (int64_t)s * r.n + c);
-        pf_l2(r.nbr + (int64_t)s * r.n + c);
-    }
+// L2 prefetch of the l-th array (l >= 0) that the rows of cells [c, c + cnt)
+// stream: the coefficients and indices of the first six slots, and the row
+// lengths.
+template <bool SYM>
+__device__ __forceinline__ void split_prefetch_rows(const BoxRows<double, SYM, false, int>& r, int l, int c, int cnt) {
+    if (l < 6 && (!SYM || (l & 1))) pf_bulk(r.val + (int64_t)l * r.n, sizeof(double), c, cnt, r.n);
+}
+template <int WIDTH, int GRP>
+__device__ __forceinline__ void split_prefetch_rows(const EllRows<double, WIDTH, int, GRP>& r, int l, int c, int cnt) {
+    const int ws = r.w < 6 ? r.w : 6;
+    if (l < ws) pf_bulk(r.val + (int64_t)l * r.n, sizeof(double), c, cnt, r.n);
+    else if (l < 2 * ws) pf_bulk(r.nbr + (int64_t)(l - ws) * r.n, sizeof(int32_t), c, cnt, r.n);
+    else if (l == 2 * ws && r.len != nullptr) pf_bulk(r.len, 1, c, cnt, r.n);
 }
 
 template <class Rows, int MINB>
@@ -4216,32 +4214,21 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_init(gf_krylov_t K,
 // applies the previous iteration's x += alpha p (it reads p_old anyway), so
 // the update kernel reads neither x nor p; x gets the same values in the
 // same order as in the other forms.
-// PF: before summing the previous kernel's partials (a chain of dependent
-// L2 reads during which HBM would idle), each thread prefetches into L2 what
-// its first PF cells will read, so the streaming starts with the kernel.
-// EARLY: in the graph loop, the prefetches that do not depend on the
-// iteration number go out before the loop's control reads, and the scalars
-// of the previous kernels (threshold, r.z, alpha) are read before the
-// partial sums instead of after them (the same values).
-template <class Rows, int MINB, bool LOOP, bool QREC = false, bool XA = false, int PF = 0, bool EARLY = false>
+// PF: warp 0 prefetches into L2, one instruction an array, the block's first
+// PF tiles before it sums the previous kernel's partials (a chain of
+// dependent L2 reads during which HBM would idle) and then tile k + PF as it
+// starts tile k.  What bounds the rows is the chain length -> index -> gather:
+// with the streams already in L2 it no longer holds an HBM round trip, four
+// blocks an SM of 64 registers (six slots' loads at once) then beat eight of
+// 32, and one tile of them ahead is 20 MB (eight blocks ahead evict what the
+// gathers need: 171 us an iteration at 4.08M cells against 146, three blocks
+// 158, two tiles 158).
+template <class Rows, int MINB, bool LOOP, bool QREC = false, bool XA = false, int PF = 0>
 __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Rows rows, int it, int pa_old,
                                                               cudaGraphConditionalHandle loop) {
     SplitScalars* S = split_scalars(K);
     const SplitVec v = split_vec(K);
     const int n = (int)K.n;
-    // early prefetch: what does not depend on the iteration number (in the
-    // graph loop this kernel never runs after the solve has stopped)
-    constexpr bool early_pf = EARLY && LOOP && PF > 0;
-    if (early_pf) {
-        const int c = blockIdx.x * blockDim.x + threadIdx.x;
-        if (c < n) {
-            pf_l2(v.z + c);
-            if (QREC) pf_l2(v.q + c);
-            if (XA) pf_l2(K.x + c);
-            pf_l2(K.diag + c);
-            split_prefetch_rows(rows, c);
-        }
-    }
     if (*(volatile int*)&S->done) {
         if (LOOP && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(loop, 0);
         return;
@@ -4251,29 +4238,14 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Ro
         pa_old = it & 1;
     }
     const bool linf = K.norm_inf != 0;
-    if (early_pf) {
-        const int c = blockIdx.x * blockDim.x + threadIdx.x;
-        if (c < n && it > 1) pf_l2((pa_old ? v.pa : v.pb) + c);
-    } else if (PF > 0) {
-        const int step = gridDim.x * blockDim.x;
-        int c = blockIdx.x * blockDim.x + threadIdx.x;
-        for (int k = 0; k < PF && c < n; ++k, c += step) {
-            pf_l2(v.z + c);
-            if (it > 1) pf_l2((pa_old ? v.pa : v.pb) + c);
-            if (QREC && it > 1) pf_l2(v.q + c);
-            if (XA && it > 1) pf_l2(K.x + c);
-            pf_l2(K.diag + c);
-            split_prefetch_rows(rows, c);
-        }
-    }
-    double e_thresh = 0.0, e_rz = 0.0, e_alpha = 0.0;
-    if (EARLY && it > 1) {
-        e_alpha = S->alpha;
-        if (threadIdx.x == 0) {
-            e_thresh = S->thresh;
-            e_rz = S->rz[(it - 1) & 1];
-        }
-    }
+    auto prefetch = [&](int c) {  // the tile that starts at cell c (warp 0)
+        const int l = threadIdx.x;
+        const double* a = l == 0 ? v.z : (l == 1 ? K.diag : (l == 2 ? (pa_old ? v.pa : v.pb) : (l == 3 ? v.q : K.x)));
+        if (l < 2 || (it > 1 && (l == 2 || (QREC && l == 3) || (XA && l == 4)))) pf_bulk(a, sizeof(double), c, kSplitThreads, n);
+        if (l >= 5) split_prefetch_rows(rows, l - 5, c, kSplitThreads);
+    };
+    if (PF > 0 && threadIdx.x < 32)
+        for (int k = 0; k < PF; ++k) prefetch((blockIdx.x + k * gridDim.x) * kSplitThreads);
     __shared__ double s_beta;
     __shared__ int s_stop;
     double red[2];
@@ -4288,14 +4260,14 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Ro
                 S->thresh = thresh;
             }
         } else {
-            thresh = EARLY ? e_thresh : S->thresh;
+            thresh = S->thresh;
         }
         int status = -1;
         if (fin < thresh) status = GF_OK;
         else if (!isfinite(fin)) status = GF_NONFINITE;
         else if (it > K.max_iter || it < 1) status = GF_MAX_ITER;
         s_stop = status >= 0;
-        s_beta = it == 1 ? 0.0 : red[1] / (EARLY ? e_rz : S->rz[(it - 1) & 1]);
+        s_beta = it == 1 ? 0.0 : red[1] / S->rz[(it - 1) & 1];
         if (blockIdx.x == 0) {
             S->fin = fin;
             if (status >= 0) {
@@ -4323,7 +4295,7 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Ro
     const double* p_old = pa_old ? v.pa : v.pb;
     // XA: x += alpha p of the previous iteration (none before the first).
     const bool upd = XA && it > 1;
-    const double alpha = upd ? (EARLY ? e_alpha : S->alpha) : 0.0;
+    const double alpha = upd ? S->alpha : 0.0;
     if (s_stop) {
         if (upd)
             for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x)
@@ -4339,6 +4311,7 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Ro
         const bool first = it == 1;
         auto gz = [&](int i) { return v.z[i]; };
         for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
+            if (PF > 0 && threadIdx.x < 32) prefetch(c - (int)threadIdx.x + PF * (int)(gridDim.x * blockDim.x));
             const double zc = v.z[c];
             const double po = first ? 0.0 : p_old[c];
             if (upd) __stcg(K.x + c, __ldcg(K.x + c) + alpha * po);
@@ -4365,30 +4338,16 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_a(gf_krylov_t K, Ro
 }
 
 // x += alpha p (not in the XA forms, whose k_cgs_a applies it); r -= alpha q;
-// z = M r; partials of |r| and r.z.
-template <int MINB, bool LOOP, bool PAIRS, bool XA = false, int PF = 0, bool EARLY = false>
+// z = M r; partials of |r| and r.z.  The tiles run from the last cell to the
+// first: k_cgs_a wrote the last q most recently and next reads the first z
+// and q, so both find part of them in L2 (4.08M cells: 145.6 us an iteration
+// in ascending order, 141.9 in descending; 1.73M: 71.4 and 70.3).  PF > 0: as
+// in k_cgs_a, for the XA forms' three arrays (4.08M: 146.5 without, 141.9).
+template <int MINB, bool LOOP, bool PAIRS, bool XA = false, int PF = 0>
 __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_b(gf_krylov_t K, int it, int p_is_b) {
     SplitScalars* S = split_scalars(K);
     const SplitVec v = split_vec(K);
     const int n = (int)K.n;
-    // the first 2 PF cells (pairs) of this thread's grid-stride loop; with
-    // EARLY in the graph loop (XA: nothing here depends on the iteration
-    // number) before the loop's control reads
-    auto prefetch = [&](int pb) {
-        const int64_t step = (int64_t)gridDim.x * blockDim.x * (PAIRS ? 2 : 1);
-        for (int64_t c = (int64_t)(blockIdx.x * blockDim.x + threadIdx.x) * (PAIRS ? 2 : 1), k = 0; k < 2 * PF && c < n;
-             ++k, c += step) {
-            pf_l2(v.r + c);
-            pf_l2(v.q + c);
-            pf_l2(K.diag + c);
-            if (!XA) {
-                pf_l2(K.x + c);
-                pf_l2((pb ? v.pb : v.pa) + c);
-            }
-        }
-    };
-    constexpr bool early_pf = EARLY && LOOP && XA && PF > 0;
-    if (early_pf) prefetch(0);
     if (*(volatile int*)&S->done) return;
     if (XA && *(volatile int*)&S->stop) {
         if (blockIdx.x == 0 && threadIdx.x == 0) S->done = 1;
@@ -4400,28 +4359,34 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_b(gf_krylov_t K, in
         if (blockIdx.x == 0 && threadIdx.x == 0) S->it_a = it + 1;
     }
     const bool jac = K.jacobi != 0, linf = K.norm_inf != 0;
-    if (PF > 0 && !early_pf) prefetch(p_is_b);
-    const double rz = EARLY ? S->rz[it & 1] : 0.0;
-    double red[1];
-    split_sum<1>(v.p1, gridDim.x, 0u, red);
-    const double alpha = (EARLY ? rz : S->rz[it & 1]) / red[0];
-    if (XA && blockIdx.x == 0 && threadIdx.x == 0) S->alpha = alpha;
-    const double* p = p_is_b ? v.pb : v.pa;
-    double loc[2] = {0.0, 0.0};
     // Pairs of cells with 16-byte loads and stores where every vector is
     // 16-byte aligned (the workspace vectors are when n is even): half the
     // memory instructions of the streaming update.
     const bool pairs = PAIRS && (n & 1) == 0 &&
                        ((reinterpret_cast<uintptr_t>(K.x) | reinterpret_cast<uintptr_t>(K.diag)) & 15u) == 0;
-    if (pairs) {
-        const int n2 = n >> 1;
-        double2* x2 = reinterpret_cast<double2*>(K.x);
-        const double2* p2 = reinterpret_cast<const double2*>(p);
-        double2* r2 = reinterpret_cast<double2*>(v.r);
-        const double2* q2 = reinterpret_cast<const double2*>(v.q);
-        double2* z2 = reinterpret_cast<double2*>(v.z);
-        const double2* d2 = reinterpret_cast<const double2*>(K.diag);
-        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += gridDim.x * blockDim.x) {
+    const int per = pairs ? 2 * kSplitThreads : kSplitThreads, tiles = (n + per - 1) / per;
+    auto prefetch = [&](int t) {
+        const int l = threadIdx.x;
+        if (t < tiles) pf_bulk(l == 0 ? v.r : (l == 1 ? v.q : K.diag), sizeof(double), (tiles - 1 - t) * per, per, n);
+    };
+    if (PF > 0 && threadIdx.x < 3)
+        for (int k = 0; k < PF; ++k) prefetch(blockIdx.x + k * gridDim.x);
+    double red[1];
+    split_sum<1>(v.p1, gridDim.x, 0u, red);
+    const double alpha = S->rz[it & 1] / red[0];
+    if (XA && blockIdx.x == 0 && threadIdx.x == 0) S->alpha = alpha;
+    const double* p = p_is_b ? v.pb : v.pa;
+    double loc[2] = {0.0, 0.0};
+    double2* x2 = reinterpret_cast<double2*>(K.x);
+    const double2* p2 = reinterpret_cast<const double2*>(p);
+    double2* r2 = reinterpret_cast<double2*>(v.r);
+    const double2* q2 = reinterpret_cast<const double2*>(v.q);
+    double2* z2 = reinterpret_cast<double2*>(v.z);
+    const double2* d2 = reinterpret_cast<const double2*>(K.diag);
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+        if (PF > 0 && threadIdx.x < 3) prefetch(t + PF * gridDim.x);
+        const int i = (tiles - 1 - t) * kSplitThreads + threadIdx.x;
+        if (pairs && 2 * i < n) {
             double2 xv = make_double2(0.0, 0.0), pv = xv;
             if (!XA) {
                 xv = __ldcg(x2 + i);
@@ -4441,14 +4406,12 @@ __global__ void __launch_bounds__(kSplitThreads, MINB) k_cgs_b(gf_krylov_t K, in
             __stcg(z2 + i, make_double2(z0, z1));
             loc[0] = norm_acc(norm_acc(loc[0], r0, linf), r1, linf);
             loc[1] += r0 * z0 + r1 * z1;
-        }
-    } else {
-        for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < n; c += gridDim.x * blockDim.x) {
-            if (!XA) __stcg(K.x + c, __ldcg(K.x + c) + alpha * __ldcg(p + c));
-            const double rk = __ldcg(v.r + c) - alpha * __ldcg(v.q + c);
-            const double zk = inv_diag(K.diag, c, jac) * rk;
-            __stcg(v.r + c, rk);
-            __stcg(v.z + c, zk);
+        } else if (!pairs && i < n) {
+            if (!XA) __stcg(K.x + i, __ldcg(K.x + i) + alpha * __ldcg(p + i));
+            const double rk = __ldcg(v.r + i) - alpha * __ldcg(v.q + i);
+            const double zk = inv_diag(K.diag, i, jac) * rk;
+            __stcg(v.r + i, rk);
+            __stcg(v.z + i, zk);
             loc[0] = norm_acc(loc[0], rk, linf);
             loc[1] += rk * zk;
         }
@@ -4578,13 +4541,13 @@ static int split_loop_exec(const void* fa, const void* fb, const gf_krylov_t& K,
     return GF_OK;
 }
 
-template <class Rows, int MINB, bool PAIRS, bool QREC = false, bool XA = false, int PF = 0, bool EARLY = false>
+template <class Rows, int MINB, bool PAIRS, bool QREC = false, bool XA = false, int PFA = 0, int PFB = 0>
 static int launch_split_rows(const gf_krylov_t* k, const Rows& rows, cudaStream_t st) {
     int dev = 0, sms = 0, per_sm = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     if (e == cudaSuccess)
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cgs_a<Rows, MINB, false, QREC, XA, PF, EARLY>, kSplitThreads, 0);
+        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_cgs_a<Rows, MINB, false, QREC, XA, PFA>, kSplitThreads, 0);
     if (e != cudaSuccess || per_sm < 1) {
         set_error("gf_pcg_solve: split CG set-up failed: %s", cudaGetErrorString(e));
         return GF_ERR_CUDA;
@@ -4616,8 +4579,8 @@ static int launch_split_rows(const gf_krylov_t* k, const Rows& rows, cudaStream_
     if (split_graph_enabled() && cudaStreamIsCapturing(st, &cap) == cudaSuccess &&
         cap == cudaStreamCaptureStatusNone) {
         cudaGraphExec_t exec = nullptr;
-        const int rc = split_loop_exec((const void*)k_cgs_a<Rows, MINB, true, QREC, XA, PF, EARLY>,
-                                       (const void*)k_cgs_b<MINB, true, PAIRS, XA, PF, EARLY>, K,
+        const int rc = split_loop_exec((const void*)k_cgs_a<Rows, MINB, true, QREC, XA, PFA>,
+                                       (const void*)k_cgs_b<MINB, true, PAIRS, XA, PFB>, K,
                                        &rows, sizeof(Rows), g, &exec);
         if (rc != GF_OK) return rc;
         e = cudaGraphLaunch(exec, st);
@@ -4629,10 +4592,10 @@ static int launch_split_rows(const gf_krylov_t* k, const Rows& rows, cudaStream_
     }
     for (int it = 1; it <= k->max_iter; ++it) {
         // p_old is pa at odd iterations (p_new then goes to pb), pb at even.
-        k_cgs_a<Rows, MINB, false, QREC, XA, PF, EARLY><<<g, kSplitThreads, 0, st>>>(K, rows, it, it & 1, 0);
-        k_cgs_b<MINB, false, PAIRS, XA, PF, EARLY><<<g, kSplitThreads, 0, st>>>(K, it, it & 1);
+        k_cgs_a<Rows, MINB, false, QREC, XA, PFA><<<g, kSplitThreads, 0, st>>>(K, rows, it, it & 1, 0);
+        k_cgs_b<MINB, false, PAIRS, XA, PFB><<<g, kSplitThreads, 0, st>>>(K, it, it & 1);
     }
-    k_cgs_a<Rows, MINB, false, QREC, XA, PF, EARLY><<<g, kSplitThreads, 0, st>>>(K, rows, k->max_iter + 1, (k->max_iter + 1) & 1, 0);
+    k_cgs_a<Rows, MINB, false, QREC, XA, PFA><<<g, kSplitThreads, 0, st>>>(K, rows, k->max_iter + 1, (k->max_iter + 1) & 1, 0);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         set_error("gf_pcg_solve: split CG launch failed: %s", cudaGetErrorString(e));
@@ -4641,7 +4604,7 @@ static int launch_split_rows(const gf_krylov_t* k, const Rows& rows, cudaStream_
     return GF_OK;
 }
 
-template <int MINB, bool PAIRS, int GRP = 1, bool QREC = false, bool XA = false, int PF = 0, bool EARLY = false>
+template <int MINB, bool PAIRS, int GRP = 1, bool QREC = false, bool XA = false, int PFA = 0, int PFB = 0>
 static int launch_split_m(const gf_krylov_t* k, void* stream) {
     const int64_t row_span = (int64_t)(k->stride_y > 0 ? 6 : (k->width > 6 ? k->width : 6)) * k->n;
     if (row_span >= ((int64_t)1 << 31)) {
@@ -4651,30 +4614,28 @@ static int launch_split_m(const gf_krylov_t* k, void* stream) {
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     if (k->stride_y > 0) {
         if (k->symmetric)
-            return launch_split_rows<BoxRows<double, true, false, int>, MINB, PAIRS, QREC, XA, PF, EARLY>(
+            return launch_split_rows<BoxRows<double, true, false, int>, MINB, PAIRS, QREC, XA, PFA, PFB>(
                 k, BoxRows<double, true, false, int>{k->val, (int)k->n, (int)k->stride_y, (int)k->stride_z}, st);
-        return launch_split_rows<BoxRows<double, false, false, int>, MINB, PAIRS, QREC, XA, PF, EARLY>(
+        return launch_split_rows<BoxRows<double, false, false, int>, MINB, PAIRS, QREC, XA, PFA, PFB>(
             k, BoxRows<double, false, false, int>{k->val, (int)k->n, (int)k->stride_y, (int)k->stride_z}, st);
     }
     // One slot at a time (the loop of a plain SpMV): the occupancy, not the
     // loads of one thread, keeps the memory system busy.
     if (k->width == 6)
-        return launch_split_rows<EllRows<double, 6, int, 1>, MINB, PAIRS, QREC, XA, PF, EARLY>(
+        return launch_split_rows<EllRows<double, 6, int, 1>, MINB, PAIRS, QREC, XA, PFA, PFB>(
             k, EllRows<double, 6, int, 1>{k->val, k->nbr, (int)k->n, k->width, k->row_len}, st);
-    return launch_split_rows<EllRows<double, 0, int, GRP>, MINB, PAIRS, QREC, XA, PF, EARLY>(
+    return launch_split_rows<EllRows<double, 0, int, GRP>, MINB, PAIRS, QREC, XA, PFA, PFB>(
         k, EllRows<double, 0, int, GRP>{k->val, k->nbr, (int)k->n, k->width, k->row_len}, st);
 }
 
 // Variant 19: 8 blocks of 256 threads an SM; 20: 6 (more registers);
 // 21: 8 with the update kernel on pairs of cells; 22: 7, pairs; 23: 7,
 // pairs, ELL slots loaded two at a time; 24: 6, pairs, four at a time;
-// 25: 8, pairs, q = A p by recurrence (the rows gather z alone); 26: 8,
-// q by recurrence, update one cell at a time; 27: 25 with x += alpha p in
-// the row kernel (the update kernel reads neither x nor p); 28: 21 with the
-// same; 29: 27 with the first cell's data prefetched into L2 while each
-// kernel sums the previous kernel's partials; 30: the same for the first two
-// cells (four of the update kernel); 31: 29 with the prefetches and the
-// scalar reads moved ahead of the loop's control reads and partial sums.
+// 25: 4, pairs, six at a time, q = A p by recurrence (the rows gather z
+// alone); 26: 8, q by recurrence, update one cell at a time; 27: 25 with
+// x += alpha p in the row kernel (the update kernel reads neither x nor p);
+// 28: 21 with the same; 29: 27 with the next tile of both kernels prefetched
+// into L2; 30: two tiles ahead in the row kernel; 31: the row kernel's alone.
 static int launch_split(const gf_krylov_t* k, void* stream, int which) {
     switch (which) {
         case 1: return launch_split_m<6, false>(k, stream);
@@ -4682,13 +4643,13 @@ static int launch_split(const gf_krylov_t* k, void* stream, int which) {
         case 3: return launch_split_m<7, true>(k, stream);
         case 4: return launch_split_m<7, true, 2>(k, stream);
         case 5: return launch_split_m<6, true, 4>(k, stream);
-        case 6: return launch_split_m<8, true, 1, true>(k, stream);
+        case 6: return launch_split_m<4, true, 6, true>(k, stream);
         case 7: return launch_split_m<8, false, 1, true>(k, stream);
-        case 8: return launch_split_m<8, true, 1, true, true>(k, stream);
+        case 8: return launch_split_m<4, true, 6, true, true>(k, stream);
         case 9: return launch_split_m<8, true, 1, false, true>(k, stream);
-        case 10: return launch_split_m<8, true, 1, true, true, 1>(k, stream);
-        case 11: return launch_split_m<8, true, 1, true, true, 2>(k, stream);
-        case 12: return launch_split_m<8, true, 1, true, true, 1, true>(k, stream);
+        case 10: return launch_split_m<4, true, 6, true, true, 1, 1>(k, stream);
+        case 11: return launch_split_m<4, true, 6, true, true, 2, 1>(k, stream);
+        case 12: return launch_split_m<4, true, 6, true, true, 1>(k, stream);
         default: return launch_split_m<8, false>(k, stream);
     }
 }

@@ -57,6 +57,17 @@ __device__ __forceinline__ double norm_acc(double acc, double r, bool linf) {
 
 __device__ __forceinline__ double norm_fin(double acc, bool linf) { return linf ? acc : sqrt(acc); }
 
+// L2 prefetch of elements [c, c + cnt) of an array of n by one instruction
+// (16-byte lines that hold at least one of them; nothing is read or faults).
+__device__ __forceinline__ void pf_bulk(const void* base, int es, int c, int cnt, int n) {
+    if (c >= n) return;
+    const int end = n - c < cnt ? n : c + cnt;
+    const uint64_t a0 = (reinterpret_cast<uint64_t>(base) + (uint64_t)c * es) & ~15ull;
+    const uint64_t a1 = (reinterpret_cast<uint64_t>(base) + (uint64_t)end * es) & ~15ull;
+    if (a1 > a0)
+        asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a0), "r"((uint32_t)(a1 - a0)) : "memory");
+}
+
 // BiCGStab per-component modes.
 enum { kDone = 0, kRun = 1, kRestart = 2, kIdle = 3, kConvS = 4 };
 

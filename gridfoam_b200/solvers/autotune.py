@@ -60,13 +60,13 @@ VARIANTS = {
     22: "split, update kernel on pairs of cells (16-byte accesses), 256 threads x 7 a SM (FP64, large systems)",
     23: "split, pairs, ELL slots loaded two at a time, 256 threads x 7 a SM (FP64, large systems)",
     24: "split, pairs, ELL slots loaded four at a time, 256 threads x 6 a SM (FP64, large systems)",
-    25: "split, pairs, q = A z + beta q by recurrence (one gathered vector), 256 threads x 8 a SM (FP64, large systems)",
+    25: "split, pairs, q = A z + beta q by recurrence (one gathered vector), six slots at a time, 256 threads x 4 a SM (FP64, large systems)",
     26: "split, q = A z + beta q by recurrence, update one cell at a time, 256 threads x 8 a SM (FP64, large systems)",
     27: "split as 25, x += alpha p in the row kernel (update kernel reads neither x nor p) (FP64, large systems)",
     28: "split as 21, x += alpha p in the row kernel (update kernel reads neither x nor p) (FP64, large systems)",
-    29: "split as 27, first cell's data prefetched into L2 while the partials are summed (FP64, large systems)",
-    30: "split as 27, first two cells' data prefetched into L2 while the partials are summed (FP64, large systems)",
-    31: "split as 29, prefetches and scalar reads ahead of the loop control reads and partial sums (FP64, large systems)",
+    29: "split as 27, next tile of both kernels prefetched into L2 by bulk instructions (FP64, large systems)",
+    30: "split as 29, two tiles ahead in the row kernel (FP64, large systems)",
+    31: "split as 29, prefetched in the row kernel alone (FP64, large systems)",
 }
 
 _LOCK = threading.Lock()

@@ -75,13 +75,12 @@ def default_variant(n: int, mixed: bool, symmetric: bool, box: bool = True) -> i
     # Above ~1.3M cells (beyond L2): the staged tiles on symmetric boxes;
     # on other rows the split CG, two plain kernels an iteration, with
     # q = A p by recurrence (the rows gather z alone), x += alpha p in the
-    # row kernel, the update kernel on pairs of cells, and each thread's
-    # first cell prefetched into L2 while the kernel sums the previous
-    # kernel's partials (fixed 100 iterations on the 4.08M-cell
-    # cylinder-wake octree: 152.4-152.7 us an iteration against 155.7-156.2
-    # without the prefetch (159.6 prefetching two cells), 158.5-159.6 with x
-    # updated in the update kernel, 163.0 with q gathered from p, 163.0 with
-    # the update one cell at a time and 164.5 for the 512-thread persistent
+    # row kernel, the update kernel on pairs of cells, and the next tile of
+    # each kernel prefetched into L2 (fixed 100 iterations on the cylinder
+    # wake's octree, us an iteration at 4.08M and 1.73M cells: 142.4 and 70.9
+    # against 157.5 and 74.9 without the prefetch, 149.3 and 79.0 for eight
+    # blocks of 32 registers an SM with the first cells prefetched; 163.0 at
+    # 4.08M with q gathered from p, 164.5 for the 512-thread persistent
     # kernel).
     return 5 if symmetric and box else 29
 
