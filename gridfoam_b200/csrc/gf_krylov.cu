@@ -5112,7 +5112,8 @@ int gf_pcg_solve(const gf_krylov_t* k, void* stream) {
         }
         if (k->variant >= kQrecVariant && k->variant <= kHaloVariant + 1) {
             int st = GF_ERR_INVALID;
-            if (k->variant >= kHaloVariant) st = launch_mixed_halo(k, stream);
+            if (k->variant == kHaloVariant) st = launch_resident(k, reinterpret_cast<cudaStream_t>(stream));
+            if (st == GF_ERR_INVALID && k->variant >= kHaloVariant) st = launch_mixed_halo(k, stream);
             if (st == GF_ERR_INVALID) st = launch_qrec(k, stream, (k->variant - kQrecVariant) % 2 == 0 ? 1 : 2);
             if (st != GF_ERR_INVALID) return st;
         }

@@ -60,7 +60,9 @@ def default_variant(n: int, mixed: bool, symmetric: bool, box: bool = True) -> i
     CG (two plain kernels an iteration, variant 29).  FP32-inner (mixed) solves: 256-thread register
     blocks below ~32K cells (6.5 us an inner iteration at 24^3, as for the
     shared-memory forms); then, up to ~1.3M cells, the single-reduction
-    form with the halo sync (6.7 against 7.0 us for the q-recurrence form
+    form with the halo sync, on boxes of up to ~300K and octrees of up to
+    ~375K cells with rows and vectors on the SMs (octree of 236K 10.5 us
+    against 14.5), else with the rows read every iteration (6.7 against 7.0 us for the q-recurrence form
     and 8.9 for the register blocks at 48^3, 7.5 against 7.8 at 64^3, 11.6
     either way at 1M cells; it falls back to the q-recurrence form where its
     six shared-memory arrays do not fit); then 512-thread blocks."""
