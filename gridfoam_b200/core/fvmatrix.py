@@ -198,10 +198,19 @@ class FvMatrix:
     # ------------------------------------------------------------------
     def _combine(self, other: "FvMatrix", a: float, b: float) -> "FvMatrix":
         res = FvMatrix(self._field, _zero=False)
-        call("gf_matrix_axpby", ctypes_ref(self._grid.cmesh), self.num_components,
-             a, ptr(self.diag_store), ptr(self.val), ptr(self.source_store),
-             b, ptr(other.diag_store), ptr(other.val), ptr(other.source_store),
-             ptr(res.diag_store), ptr(res.val), ptr(res.source_store), stream_ptr())
+        if self.num_components in (1, 3):
+            call("gf_matrix_axpby", ctypes_ref(self._grid.cmesh), self.num_components,
+                 a, ptr(self.diag_store), ptr(self.val), ptr(self.source_store),
+                 b, ptr(other.diag_store), ptr(other.val), ptr(other.source_store),
+                 ptr(res.diag_store), ptr(res.val), ptr(res.source_store), stream_ptr())
+        else:  # the one-pass kernel has instances for one and three components
+            s = stream_ptr()
+            for x, y, out in (
+                (self.diag_store, other.diag_store, res.diag_store),
+                (self.val, other.val, res.val),
+                (self.source_store, other.source_store, res.source_store),
+            ):
+                call("gf_axpby", x.numel(), a, ptr(x), b, ptr(y), ptr(out), s)
         res._ffc = self._combine_ffc(self._ffc, other._ffc, a, b)
         if self.requires_grad or other.requires_grad:
             xs, ys = self.autograd_tensors(), other.autograd_tensors()
