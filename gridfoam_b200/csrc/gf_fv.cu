@@ -478,10 +478,17 @@ __global__ void __launch_bounds__(kLsqThreads) k_lsq_list(gf_mesh_t m, int64_t n
     if (i < n) lsq_any_cell<NC>(m, __ldg(cells + i), psi, kind, psib, grad);
 }
 
-// Cells from which the regular cells get a kernel of their own.  Below, a
-// gradient takes about 10 us either way, and the general kernel keeps the
-// bits that the distances between rounded cell centres give.
-constexpr int64_t kRegularCells = 131072;
+// Cells from which the regular cells get a kernel of their own: where a pass
+// of explicit operators stops being bound by its launches.  The two kernels
+// are the faster on the device at every size (three components, 135K cells of
+// a box 10.5 us against 11.4, 301K 13.1 against 27.1), but they are one launch
+// more a gradient, and up to some 300K cells that is what the pass waits for:
+// boxes of 205K cells 138 us a pass against 132, 278K 137 against 130, 301K
+// 139 against 132, octrees of 196K 183 against 175, 279K 184 against 177; then
+// boxes of 363K 138 against 149, 512K 144 against 197, octrees of 369K 183
+// against 206.  Below, the general kernel also keeps the bits that the
+// distances between rounded cell centres give.
+constexpr int64_t kRegularCells = 327680;
 
 static bool has_regular(const gf_mesh_t* m) {
     return m->reg_level != nullptr && (m->irr_cells != nullptr || m->n_irr == 0) && m->n_cells >= kRegularCells &&
