@@ -4782,10 +4782,15 @@ static int launch_staged(const gf_krylov_t* k, int T, void* stream) {
     const char* what = "gf_pcg_solve";
     const void* kern = (const void*)k_pcg1_box_staged<kStThreads>;
     const size_t smem = (size_t)2 * StLayout(T, k->stride_y).stage() * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    int dev = 0, sms = 0, per_sm = 0;
-    if (e == cudaSuccess) e = cudaGetDevice(&dev);
+    int dev = 0, sms = 0, per_sm = 0, optin = 0;
+    cudaFuncAttributes fa = {};
+    cudaError_t e = cudaGetDevice(&dev);
     if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kern);
+    // always the most a block can have (see launch_smem_arrays)
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kStThreads, smem);
     if (e != cudaSuccess || per_sm < 1) {
         set_error("%s: staged kernel set-up failed: %s", what, cudaGetErrorString(e));
@@ -5008,7 +5013,10 @@ static int launch_smem_arrays(const gf_krylov_t* k, void* stream, int threads, i
         chunk = (chunk + 1) & ~1LL;
         const size_t smem = (size_t)(narr * chunk) * elem;
         if ((int64_t)smem + static_smem > optin) continue;
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        // The attribute is the kernel's, not the launch's: always the most a
+        // block can have, so that threads with systems of other sizes do not
+        // take it below what this launch needs.
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(optin - static_smem));
         int occ = 0;
         if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kSmemThreads, smem);
         if (e != cudaSuccess) {

@@ -564,7 +564,10 @@ int launch_resident(const gf_krylov_t* k, cudaStream_t st) {
     const void* kern = mixed ? (wide ? res_mixed_kernel<true>(u) : res_mixed_kernel<false>(u))
                              : (wide ? res_kernel<true>(u) : res_kernel<false>(u));
     int occ = 0;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    // The attribute is the kernel's, not the launch's: set to the same bound by
+    // every caller, or a thread with a smaller system would take it below what
+    // another is about to launch with.
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)room);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, kRT, smem);
     if (e == cudaSuccess && (int64_t)occ * sms < grid) return GF_ERR_INVALID;
     if (e == cudaSuccess) e = cudaMemsetAsync(k->work, 0, sizeof(KCtl), st);
