@@ -5233,12 +5233,12 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream) {
         }
     }
     if (!valid_krylov(k, 6, "gf_bicgstab_solve", k ? k->n : 0)) return GF_ERR_INVALID;
-    if (k->stride_y > 0 && (k->width != 6 || k->stride_z < k->stride_y)) {
-        set_error("gf_bicgstab_solve: a box layout needs width 6 and strides 1 <= stride_y <= stride_z");
-        return GF_ERR_INVALID;
-    }
-    if (cluster_fits(*k, true)) return launch_cluster(k, true, reinterpret_cast<cudaStream_t>(stream));
-    return launch_persistent(bicgstab_kernel(*k), k, stream, "gf_bicgstab_solve", kBicgThreads);
+    gf_krylov_t q = *k;
+    // Strides that no box layout has (CG refuses them): by the index table,
+    // which says the same and is given in every case.
+    if (q.stride_y < 1 || q.width != 6 || q.stride_z < q.stride_y) q.stride_y = q.stride_z = 0;
+    if (cluster_fits(q, true)) return launch_cluster(&q, true, reinterpret_cast<cudaStream_t>(stream));
+    return launch_persistent(bicgstab_kernel(q), &q, stream, "gf_bicgstab_solve", kBicgThreads);
 }
 
 }  // extern "C"

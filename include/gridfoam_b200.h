@@ -227,7 +227,9 @@ typedef struct gf_krylov {
     double inner_eta;     /* inner FP32 cycle stops at eta * |r_true| */
     int64_t stride_y;     /* > 0: the ELL is a uniform lexicographic box with
                              slots -x,+x,-y,+y,-z,+z, so neighbours are
-                             c -+ 1, c -+ stride_y, c -+ stride_z (nbr unread) */
+                             c -+ 1, c -+ stride_y, c -+ stride_z (nbr unread).
+                             Rows of another width or stride_z < stride_y:
+                             refused by CG; BiCGStab goes by nbr */
     int64_t stride_z;
     int32_t symmetric;    /* 1 (box only): A is symmetric, only + slots read */
     int32_t block_cap;    /* > 0: at most this many persistent blocks (tuning) */
