@@ -38,7 +38,8 @@ __global__ void __launch_bounds__(128) k_bc_state(gf_mesh_t m, gf_bc_t bc, const
         double psiP[3], value[3], refv[3] = {0, 0, 0}, refg[3] = {0, 0, 0};
 #pragma unroll
         for (int k = 0; k < nc; ++k) {
-            value[k] = __ldg(bc.value + k * nb + b);
+            // before the kind is known; a table of kinds that need none may have none
+            value[k] = bc.value != nullptr ? __ldg(bc.value + k * nb + b) : 0.0;
             psiP[k] = psi[k * C + c];
         }
         double frac = 0.0;

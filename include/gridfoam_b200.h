@@ -144,7 +144,8 @@ typedef struct gf_bc {
     int32_t reserved;
     const int8_t* kind;    /* [Nb] GF_BC_* */
     const double* value;   /* [ncomp][Nb] Dirichlet value / Neumann gradient /
-                              inletOutlet reverse-inflow value */
+                              inletOutlet reverse-inflow value; NULL where
+                              no face has one of these kinds */
 } gf_bc_t;
 
 /* Evaluated boundary state (fv/boundary_ops.py:311-326). */
