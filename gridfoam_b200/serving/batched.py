@@ -85,9 +85,13 @@ class _Case:
         sim = cavity_simulator(req.nu, req.lid, p_tol=engine.p_tol, p_solver_tol=engine.p_solver_tol,
                                p_solver_rtol=engine.p_solver_rtol, max_outer=engine.max_outer,
                                inner_precision=engine.inner_precision, device=str(engine.device.type))
-        with torch.cuda.stream(self.stream):
-            self.algo = create_algorithm(engine.topologies.grid(req.n, sim))
-            self.algo.set_host_readback(False)
+        try:
+            with torch.cuda.stream(self.stream):
+                self.algo = create_algorithm(engine.topologies.grid(req.n, sim))
+                self.algo.set_host_readback(False)
+        except BaseException:
+            engine._keep_stream(self)
+            raise
         self.cg_blocks = blocks_for(req.n**3, False)
         self.bicg_blocks = blocks_for(req.n**3, True)
 
@@ -183,11 +187,14 @@ class BatchedEngine:
                 del slot
             else:
                 case = _Case(self, req, 0.0)
-                self._iteration([case], capture=False)
-                torch.cuda.synchronize(self.device)
-                used = torch.cuda.memory_allocated(self.device) - before
-                case.release()
-                self._keep_stream(case)
+                try:
+                    self._iteration([case], capture=False)
+                    torch.cuda.synchronize(self.device)
+                    used = torch.cuda.memory_allocated(self.device) - before
+                finally:
+                    torch.cuda.synchronize(self.device)  # the engine's stream too, before the memory goes
+                    case.release()
+                    self._keep_stream(case)
             self.footprint[n] = int(1.1 * used) + (1 << 20)
 
     def is_solo(self, n: int) -> bool:
@@ -276,7 +283,9 @@ class BatchedEngine:
         return graph
 
     def _keep_stream(self, c: _Case) -> None:
-        """Keep a finished case's stream (synchronised) for the next one."""
+        """Keep the stream of a case that is finished, or could not be built,
+        for the next one.  What is still queued on it runs before the next
+        case's work, and memory freed by the case serves that stream alone."""
         if len(self._streams) < self.MAX_SLOTS:
             self._streams.append(c.stream)
 
@@ -362,6 +371,7 @@ class BatchedEngine:
                             continue
                     queue.remove(req)
                     admitted = True
+                    case = None
                     try:
                         if self.admission_hook is not None:
                             self.admission_hook(req)
@@ -370,6 +380,9 @@ class BatchedEngine:
                             self.case_hook(case)
                     except (RuntimeError, ValueError, torch.cuda.OutOfMemoryError) as exc:
                         results.append(self._reject(req, now(), f"rejected: {type(exc).__name__}"))
+                        if isinstance(case, _Case):  # built, then refused by the hook
+                            case.release()
+                            self._keep_stream(case)
                         break
                     case.need = need
                     used += need
