@@ -122,6 +122,7 @@ class BatchedEngine:
     """
 
     MAX_SLOTS = 16
+    CAPTURE_ROOM = 64 << 20  # free device bytes a capture wants (it takes one 2 MB segment)
 
     def __init__(self, device="cuda", *, hbm_budget: int | None = None, max_slots: int = 8,
                  use_graphs: bool = True, p_tol: float = 1e-6, p_solver_tol: float = 1e-12,
@@ -270,9 +271,13 @@ class BatchedEngine:
         would also collect garbage and empty the allocator's cache, and the
         next cases' some forty tensors each would go to the driver again
         (0.1 to 0.8 ms a tensor): with both, eight cavities of ten outer
-        iterations took 64 to 120 ms, without 42.  The iteration allocates
-        nothing that would need the room."""
+        iterations took 64 to 120 ms, without 42.  The iteration allocates a
+        few small tensors in the graph's own pool; where the device has no
+        room for one more segment, the cache goes first, since the allocator
+        cannot give it back during a capture."""
         torch.cuda.synchronize(self.device)
+        if torch.cuda.mem_get_info(self.device)[0] < self.CAPTURE_ROOM:
+            torch.cuda.empty_cache()
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.stream(self.stream):
             graph.capture_begin()

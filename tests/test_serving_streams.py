@@ -74,3 +74,16 @@ def test_a_lone_failing_case_leaves_the_streams_as_they_were(monkeypatch):
         (r,) = eng.run(_mix()[:1])
     assert r.status == "rejected: RuntimeError"
     assert [id(s) for s in eng._streams] == before
+
+
+@pytest.mark.parametrize("free,emptied", [(1 << 20, True), (1 << 33, False)])
+def test_a_capture_on_a_full_device_empties_the_allocators_cache(free, emptied, monkeypatch):
+    """The allocator cannot give cached blocks back during a capture."""
+    eng = _engine()
+    calls = []
+    empty = torch.cuda.empty_cache
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda *a: (free, 1 << 37))
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: (calls.append(1), empty()))
+    (r,) = eng.run(_mix()[:1])
+    assert r.iterations == 6 and eng.captures > 0
+    assert bool(calls) == emptied
