@@ -208,6 +208,7 @@ _SIGNATURES = {
     "gf_pcg_solve_batched": ([P, I32, P, P], ctypes.c_int),
     "gf_bicgstab_solve_batched": ([P, I32, P, P], ctypes.c_int),
     "gf_batch_max_blocks": ([I32], ctypes.c_int),
+    "gf_bicgstab_max_blocks": ([I32, I32, I32], ctypes.c_int),
     "gf_rau_hbya": ([P, I32, P, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_simplec_rAtU": ([P, P, P, P, P], ctypes.c_int),
     "gf_face_flux": ([P, I32, P, P, P, P, P, P, P], ctypes.c_int),

@@ -5047,6 +5047,15 @@ static int launch_smem_arrays(const gf_krylov_t* k, void* stream, int threads, i
 }
 
 // nvec vectors of ncomp x n doubles plus `extra` doubles after the header.
+template <int WIDTH>
+static const void* bi_mixed_kernel(int ncomp) {
+    return ncomp == 1 ? (const void*)k_bicgstab_mixed<1, WIDTH>
+                      : (ncomp == 2 ? (const void*)k_bicgstab_mixed<2, WIDTH> : (const void*)k_bicgstab_mixed<3, WIDTH>);
+}
+static const void* bicgstab_mixed_kernel(int ncomp, int width) {
+    return width == 6 ? bi_mixed_kernel<6>(ncomp) : bi_mixed_kernel<0>(ncomp);
+}
+
 static bool valid_krylov(const gf_krylov_t* k, int nvec, const char* what, int64_t extra = 0) {
     if (k == nullptr || k->n <= 0 || k->width <= 0 || k->ncomp < 1 || k->ncomp > 3 || k->nbr == nullptr ||
         k->diag == nullptr || k->val == nullptr || k->rhs == nullptr || k->x == nullptr || k->work == nullptr ||
@@ -5219,18 +5228,7 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream) {
                       "BiCGStab workspace", kMaxEll);
             return GF_ERR_INVALID;
         }
-        const bool m6 = k->width == 6;
-        switch (k->ncomp) {
-            case 1:
-                return m6 ? launch_persistent(k_bicgstab_mixed<1, 6>, k, stream, "gf_bicgstab_solve")
-                          : launch_persistent(k_bicgstab_mixed<1, 0>, k, stream, "gf_bicgstab_solve");
-            case 2:
-                return m6 ? launch_persistent(k_bicgstab_mixed<2, 6>, k, stream, "gf_bicgstab_solve")
-                          : launch_persistent(k_bicgstab_mixed<2, 0>, k, stream, "gf_bicgstab_solve");
-            default:
-                return m6 ? launch_persistent(k_bicgstab_mixed<3, 6>, k, stream, "gf_bicgstab_solve")
-                          : launch_persistent(k_bicgstab_mixed<3, 0>, k, stream, "gf_bicgstab_solve");
-        }
+        return launch_persistent(bicgstab_mixed_kernel(k->ncomp, k->width), k, stream, "gf_bicgstab_solve");
     }
     if (!valid_krylov(k, 6, "gf_bicgstab_solve", k ? k->n : 0)) return GF_ERR_INVALID;
     gf_krylov_t q = *k;
@@ -5343,6 +5341,25 @@ int gf_batch_max_blocks(int32_t bicgstab) {
         cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bicgstab ? kKThreads : kCgThreads,
                                                                       0) != cudaSuccess) {
         set_error("gf_batch_max_blocks: device query failed");
+        return -1;
+    }
+    return per_sm * sms;
+}
+
+int gf_bicgstab_max_blocks(int32_t ncomp, int32_t width, int32_t mixed) {
+    if (ncomp < 1 || ncomp > 3 || width < 1) {
+        set_error("gf_bicgstab_max_blocks: 1 to 3 components and rows of at least one slot");
+        return -1;
+    }
+    gf_krylov_t k = {};
+    k.ncomp = ncomp;
+    k.width = width;
+    const void* kern = mixed ? bicgstab_mixed_kernel(ncomp, width) : bicgstab_kernel(k);
+    int dev = 0, sms = 0, per_sm = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) !=
+        cudaSuccess || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, mixed ? kKThreads : kBicgThreads,
+                                                                      0) != cudaSuccess) {
+        set_error("gf_bicgstab_max_blocks: device query failed");
         return -1;
     }
     return per_sm * sms;

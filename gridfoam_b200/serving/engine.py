@@ -34,8 +34,10 @@ from dataclasses import dataclass, field
 import numpy as np
 import torch
 
+from gridfoam_b200._lib import load
 from gridfoam_b200.serving.cases import TopologyCache, cavity_simulator
 from gridfoam_b200.serving.requests import CavityRequest
+from gridfoam_b200.solvers.krylov import default_variant
 
 
 @dataclass
@@ -56,9 +58,25 @@ class ServeResult:
         return self.finished - self.arrival
 
 
-# Resident blocks per SM of the persistent CG launch shapes (variants 0-5)
-# and of BiCGStab; a slot's block cap is a share of these.
+# Resident blocks per SM of the persistent CG launch shapes (variants 0-5; one
+# for the others, or more): a slot's block cap is a share of these.
 _BLOCKS_PER_SM = {0: 4, 1: 4, 2: 2, 3: 1, 4: 1, 5: 1}
+
+
+def block_cap(solver, n: int, ncomp: int, width: int, share: float, sms: int, bicgstab_blocks) -> int:
+    """Blocks that a slot's solver may take for its share of the GPU: of the
+    blocks of the kernel that it will run that fit on the GPU at once.
+    ``bicgstab_blocks(ncomp, width, mixed)`` gives them for BiCGStab (one an
+    SM in both precisions, 1024 threads or 512 of 128 registers); the CG's
+    follow from its launch shape, the default one for the size included."""
+    if solver.bicgstab:
+        blocks = bicgstab_blocks(ncomp, width, int(solver.mixed))
+    else:
+        v = solver.variant
+        if v is None:
+            v = default_variant(n, solver.mixed, True)
+        blocks = sms * _BLOCKS_PER_SM.get(v, 1)
+    return max(1, int(share * blocks))
 
 
 class _Slot:
@@ -90,9 +108,9 @@ class _Slot:
                 self.algo.solvers["p"].variant = variant
             if engine.gpu_share < 1.0:
                 for name, s in self.algo.solvers.items():
-                    v = s.variant if s.variant is not None else 0
-                    per_sm = 2 if s.bicgstab else _BLOCKS_PER_SM.get(v, 1)
-                    s.block_cap = max(1, int(engine.gpu_share * engine.sms * per_sm))
+                    nc = self.algo.U.num_components if name == self.algo.U.name else 1
+                    s.block_cap = block_cap(s, grid.num_cells, nc, grid.ell_width, engine.gpu_share, engine.sms,
+                                            load().gf_bicgstab_max_blocks)
             self.res_host = torch.empty(1, dtype=torch.float64, pin_memory=True)
             self.event = torch.cuda.Event()
             # First iteration eagerly: allocates every workspace and cache.

@@ -339,6 +339,9 @@ int64_t gf_pcg_static_scratch_doubles(void);
 /* solvers/bicgstab.py:76-272: right-preconditioned BiCGStab with breakdown
  * restarts, one persistent cooperative launch, ncomp systems at once. */
 int gf_bicgstab_solve(const gf_krylov_t* k, void* stream);
+/* Co-resident blocks of the grid BiCGStab kernel for these systems on the
+ * current device (what a block_cap is a share of), or -1. */
+int gf_bicgstab_max_blocks(int32_t ncomp, int32_t width, int32_t mixed);
 
 /* Batched solves for the solve server (no counterpart in the reference,
  * which solves one case at a time, solvers/krylov.py:34-82): the systems of
