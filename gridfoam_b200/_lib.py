@@ -195,6 +195,7 @@ _SIGNATURES = {
     "gf_krylov_workspace_size": ([I64, I32, I32], I64),
     "gf_bc_state": ([P, P, P, P, P, P], ctypes.c_int),
     "gf_lsq_grad": ([P, I32, P, P, P, P, P], ctypes.c_int),
+    "gf_lsq_grad_launches": ([P], ctypes.c_int),
     "gf_lsq_grad_hang": ([P, I32, P, P, P, P, P], ctypes.c_int),
     "gf_assemble": ([P, P, P], ctypes.c_int),
     "gf_momentum_finalize": ([P, I32, F64, P, P, P, P, P, P], ctypes.c_int),
@@ -209,6 +210,7 @@ _SIGNATURES = {
     "gf_bicgstab_solve_batched": ([P, I32, P, P], ctypes.c_int),
     "gf_batch_max_blocks": ([I32], ctypes.c_int),
     "gf_bicgstab_max_blocks": ([I32, I32, I32], ctypes.c_int),
+    "gf_split_loop_unroll": ([], ctypes.c_int),
     "gf_rau_hbya": ([P, I32, P, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_simplec_rAtU": ([P, P, P, P, P], ctypes.c_int),
     "gf_face_flux": ([P, I32, P, P, P, P, P, P, P], ctypes.c_int),
@@ -278,12 +280,35 @@ class GfError(RuntimeError):
     """A gridfoam_b200 library call failed."""
 
 
-# Kernels launched per entry point (for launch accounting).
+def _grad_launches(args) -> int:
+    """A gradient's launches, asked once a mesh descriptor (``args[0]`` is a
+    ``byref`` of it)."""
+    m = args[0]._obj
+    n = getattr(m, "grad_launches", 0)
+    if not n:
+        n = m.grad_launches = load().gf_lsq_grad_launches(args[0])
+    return n
+
+
+def _hang_grad_launches(args) -> int:
+    m = args[0]._obj
+    return int(m.n_hang_cells > 0) if m.hang_cells else _grad_launches(args)
+
+
+def _face_flux_launches(args) -> int:
+    """Axis-aligned internal faces and the boundary faces apart, or all in one."""
+    m = args[0]._obj
+    return 1 + int(bool(m.face_axis) and m.n_faces > 0 and m.n_bnd > 0)
+
+
+# Kernels launched per entry point (for launch accounting): a number, or a
+# function of the call's arguments.
 _LAUNCHES_PER_CALL = {"gf_fixed_values": 3, "gf_close_fixed_flux": 2, "gf_field_residual": 2, "gf_continuity_sums": 2,
-                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2}
+                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2, "gf_lsq_grad": _grad_launches,
+                      "gf_lsq_grad_hang": _hang_grad_launches, "gf_face_flux": _face_flux_launches}
 LAUNCHES: collections.Counter = collections.Counter()
-# Launches known only after the device ran (the split CG's graph loop runs
-# two kernels an iteration): callables giving their counts, kept while
+# Launches known only after the device ran (the split CG's graph loop, whole
+# bodies of some iterations): callables giving their counts, kept while
 # TRACK_DEFERRED is set (see ``launch_total``).
 TRACK_DEFERRED = False
 DEFERRED_LAUNCHES: list = []
@@ -303,7 +328,8 @@ def call(name: str, *args) -> int:
     """Call ``name`` and raise :class:`GfError` on a non-zero status."""
     lib = load()
     status = getattr(lib, name)(*args)
-    LAUNCHES[name] += _LAUNCHES_PER_CALL.get(name, 1)
+    per = _LAUNCHES_PER_CALL.get(name, 1)
+    LAUNCHES[name] += per if per.__class__ is int else per(args)
     if status != GF_OK:
         msg = lib.gf_last_error().decode(errors="replace")
         raise GfError(f"{name} failed with status {status}: {msg}")

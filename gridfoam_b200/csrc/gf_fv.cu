@@ -2008,6 +2008,8 @@ int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8
     return check_launch("gf_lsq_grad");
 }
 
+int gf_lsq_grad_launches(const gf_mesh_t* m) { return m != nullptr && has_regular(m) && m->n_irr > 0 ? 2 : 1; }
+
 int gf_lsq_grad_hang(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8_t* bc_kind, const double* psib,
                      double* grad, void* stream) {
     if (!valid_mesh(m) || !valid_nc(ncomp) || m->lsq_ata_inv == nullptr) return GF_ERR_INVALID;

@@ -5346,6 +5346,8 @@ int gf_batch_max_blocks(int32_t bicgstab) {
     return per_sm * sms;
 }
 
+int gf_split_loop_unroll(void) { return kSplitUnroll; }
+
 int gf_bicgstab_max_blocks(int32_t ncomp, int32_t width, int32_t mixed) {
     if (ncomp < 1 || ncomp > 3 || width < 1) {
         set_error("gf_bicgstab_max_blocks: 1 to 3 components and rows of at least one slot");

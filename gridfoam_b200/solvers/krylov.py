@@ -151,8 +151,10 @@ class DeviceKrylov(LinearSolver):
         buf = _StatsBuffer(stats)
         out = tuple(SolveStats(self.solver_name, buf, i) for i in range(nc))
         if graph_loop and _lib.TRACK_DEFERRED:
-            # the graph loop runs its two kernels iterations + 1 times
-            _lib.DEFERRED_LAUNCHES.append(lambda st=out[0]: 2 * (st.iterations + 1))
+            # two kernels for every iteration and the one that finds the stop,
+            # in whole bodies of the loop
+            u = load().gf_split_loop_unroll()
+            _lib.DEFERRED_LAUNCHES.append(lambda st=out[0]: 2 * u * -(-(st.iterations + 1) // u))
         if ev is not None:
             self.profile_events.append((ev[0], ev[1], out))
         return out

@@ -272,6 +272,8 @@ int gf_bc_state(const gf_mesh_t* m, const gf_bc_t* bc, const double* psi,
 int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi,
                 const int8_t* bc_kind, const double* psib, double* grad,
                 void* stream);
+/* Kernels that gf_lsq_grad launches on this mesh. */
+int gf_lsq_grad_launches(const gf_mesh_t* m);
 
 /* The same gradient at the cells with a hanging face only (mesh hang_cells;
  * everywhere when that is NULL): all that the hanging-face corrections of
@@ -342,6 +344,9 @@ int gf_bicgstab_solve(const gf_krylov_t* k, void* stream);
 /* Co-resident blocks of the grid BiCGStab kernel for these systems on the
  * current device (what a block_cap is a share of), or -1. */
 int gf_bicgstab_max_blocks(int32_t ncomp, int32_t width, int32_t mixed);
+/* Iterations (two kernels each) in the body of the split CG's graph loop:
+ * a body that holds the stop is launched whole. */
+int gf_split_loop_unroll(void);
 
 /* Batched solves for the solve server (no counterpart in the reference,
  * which solves one case at a time, solvers/krylov.py:34-82): the systems of
