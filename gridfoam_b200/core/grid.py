@@ -172,8 +172,6 @@ class AxisProjectedGrid:
         move_o[hidx, axis[hang_faces]] = 0.0
         move_n[hidx, axis[hang_faces]] = 0.0
 
-        reg_h, reg_level = self._regular_cells(centers, sizes, owner, neighbour, axis, d_all, immersed, dom_owner)
-
         # Boundary faces: domain | immersed upper | immersed lower
         iSf = Sf[imm_faces]
         i_mag = np.linalg.norm(iSf, axis=1) if Fi else np.zeros(0)
@@ -245,8 +243,6 @@ class AxisProjectedGrid:
         normals = getattr(ap, "anchor_normal", None)
         host.extra["anchor_normal"] = (np.asarray(normals, dtype=np.float64).reshape(Fi, 3)
                                        if normals is not None else None)
-        host.extra["reg_h"] = reg_h
-        host.extra["reg_level"] = reg_level
         host.extra["hang_cells"] = np.unique(np.concatenate([owner[hang_faces], neighbour[hang_faces]]))
         host.extra["hang_faces"] = hang_faces
         host.extra["hang_offset"] = hang_offset
@@ -254,25 +250,31 @@ class AxisProjectedGrid:
         host.extra["hang_move_n"] = move_n
         return host
 
-    @staticmethod
-    def _regular_cells(centers, sizes, owner, neighbour, axis, d_all, immersed, dom_owner):
+    def _regular_cells(self) -> tuple[torch.Tensor, torch.Tensor]:
         """``(h [3], level [C] uint8)``: cells whose six faces are internal,
         not immersed and lead to cells of their own size ``h 2^level`` at
         that distance along the axes; 255 for the others.  Their geometry
-        follows from the level, so the kernels need not read it."""
-        C = sizes.shape[0]
-        h = sizes.min(axis=0)
-        level = np.rint(np.log2(sizes[:, 0] / h[0]))
-        ok = (level < 32) & (sizes == h * np.exp2(level)[:, None]).all(axis=1)
-        fidx = np.arange(owner.shape[0])
-        d_n = np.abs(d_all[fidx, axis])
-        want = h[axis] * np.exp2(level[owner])
-        same = (ok[owner] & ok[neighbour] & (level[owner] == level[neighbour]) & ~immersed
-                & (np.abs(d_n - want) <= 1e-9 * want) & (np.abs(d_all).sum(axis=1) - d_n <= 1e-9 * want))
-        faces = np.bincount(owner, minlength=C) + np.bincount(neighbour, minlength=C)
-        faces += np.bincount(dom_owner, minlength=C)
-        regular = np.bincount(owner[same], minlength=C) + np.bincount(neighbour[same], minlength=C)
-        return h, np.where(ok & (faces == 6) & (regular == 6), level, 255).astype(np.uint8)
+        follows from the level, so the kernels need not read it.  On the
+        device: with numpy it took 0.26 s of the 3.7 s set-up of 96^3 cells."""
+        owner, neighbour, axis, C = self._owner, self._neighbour, self._axis, self._num_cells
+        center, sizes = self.dev["center"], self._cell_sizes
+        h = sizes.amin(0)
+        level = torch.round(torch.log2(sizes[:, 0] / h[0])).clamp(0, 32).long()
+        scale = torch.tensor([2.0**i for i in range(33)], dtype=torch.float64, device=sizes.device)[level]
+        ok = (level < 32) & (sizes == h * scale[:, None]).all(1)
+        want = h[axis] * scale[owner]
+        along, off = torch.zeros_like(want), torch.zeros_like(want)
+        for a in range(3):
+            d = (center[a][neighbour] - center[a][owner]).abs()
+            on = axis == a
+            along += d * on
+            off += d * ~on
+        same = (ok[owner] & ok[neighbour] & (level[owner] == level[neighbour]) & ~self._ap_is_immersed_faces
+                & ((along - want).abs() <= 1e-9 * want) & (off <= 1e-9 * want))
+        count = lambda cells: torch.bincount(cells, minlength=C)  # noqa: E731
+        faces = count(owner) + count(neighbour) + count(self._domain_bnd_owner)
+        regular = count(owner[same]) + count(neighbour[same])
+        return h, torch.where(ok & (faces == 6) & (regular == 6), level, 255).to(torch.uint8)
 
     def _build_ell(self) -> None:
         """Cell-centric slot table sorted by (cell, direction, face).
@@ -391,8 +393,6 @@ class AxisProjectedGrid:
             "face_pos_neigh": i32(h.extra["face_pos_neigh"]),
             "face_axis": torch.as_tensor(np.ascontiguousarray(h.axis, dtype=np.int8), device=dev),
         }
-        t["reg_level"] = torch.as_tensor(h.extra["reg_level"], device=dev)
-        t["irr_cells"] = i32(np.nonzero(h.extra["reg_level"] == 255)[0])
         hf = h.extra["hang_faces"]
         face_hang = np.full(self._num_internal_faces, -1, dtype=np.int64)
         face_hang[hf] = np.arange(hf.shape[0])
@@ -404,22 +404,6 @@ class AxisProjectedGrid:
             t["hang_move_o"] = f64(h.extra["hang_move_o"].T)
             t["hang_move_n"] = f64(h.extra["hang_move_n"].T)
         self.dev = t
-        m = GfMesh()
-        m.n_cells = self._num_cells
-        m.n_faces = self._num_internal_faces
-        m.n_domain = self._num_domain_bnd_faces
-        m.n_imm = self._num_immersed_faces
-        m.n_bnd = self.num_bnd
-        m.ell_width = self._ell_width
-        m.n_hang = int(hf.shape[0])
-        m.n_irr = int(t["irr_cells"].numel())
-        m.n_hang_cells = int(h.extra["hang_cells"].shape[0])
-        m.reg_h = tuple(float(v) for v in h.extra["reg_h"])
-        if self.box_strides is not None:
-            m.stride_y, m.stride_z = self.box_strides
-        for name, tensor in t.items():
-            setattr(m, name, ptr(tensor))
-        self.cmesh = m
         # Reference-layout tensors for the public accessors.
         self._owner = i64(h.owner)
         self._neighbour = i64(h.neighbour)
@@ -433,6 +417,24 @@ class AxisProjectedGrid:
         self._domain_bnd_face_centers = f64(h.domain_face_centers)
         self._domain_bnd_Sf = f64(h.domain_Sf)
         self._ap_is_immersed_faces = torch.as_tensor(h.immersed, device=dev)
+        reg_h, t["reg_level"] = self._regular_cells()
+        t["irr_cells"] = torch.nonzero(t["reg_level"] == 255).reshape(-1).to(torch.int32)
+        m = GfMesh()
+        m.n_cells = self._num_cells
+        m.n_faces = self._num_internal_faces
+        m.n_domain = self._num_domain_bnd_faces
+        m.n_imm = self._num_immersed_faces
+        m.n_bnd = self.num_bnd
+        m.ell_width = self._ell_width
+        m.n_hang = int(hf.shape[0])
+        m.n_irr = int(t["irr_cells"].numel())
+        m.n_hang_cells = int(h.extra["hang_cells"].shape[0])
+        m.reg_h = tuple(reg_h.tolist())
+        if self.box_strides is not None:
+            m.stride_y, m.stride_z = self.box_strides
+        for name, tensor in t.items():
+            setattr(m, name, ptr(tensor))
+        self.cmesh = m
         self.single_idx = i64(np.nonzero(~h.immersed)[0])
         self.single_is_identity = self._num_immersed_faces == 0
 
