@@ -1,7 +1,8 @@
 // FP64 BiCGStab on the whole grid (sm_100a): one persistent cooperative
 // launch for up to three components that share the matrix reads, for systems
-// beyond what a cluster holds (gf_cluster.cu), and the batched form that
-// gives each system a share of the blocks.
+// beyond what a cluster holds (gf_cluster.cu) and for callers that bound the
+// blocks or the waits.  (The batched form, which gives each system a share of
+// the blocks, is in gf_krylov.cu.)
 //
 // The reference's right-preconditioned BiCGStab (bicgstab.py:76-272), its
 // breakdown tests and restarts included, in five passes over the cells:

@@ -551,8 +551,8 @@ bool cluster_fits(const gf_krylov_t& k, bool bicgstab) {
     if (k.mixed || k.single_reduction || k.block_cap > 0 || k.spin_limit > 0) return false;
     if (!bicgstab && k.ncomp != 1) return false;
     // The largest system: its rows (80 bytes a cell at width 6) in 16 blocks'
-    // shared memory and its vectors in their registers, up to 43,000 cells for
-    // the CG and 32,768 for BiCGStab.  There the cluster is still the faster
+    // shared memory and its vectors in their registers, up to 44,816 cells for
+    // the CG (2,801 a block) and 32,768 for BiCGStab.  There the cluster is still the faster
     // (CG 4.6 against 6.8 us at 42,875 cells, BiCGStab 9.6 against 43).
     const int64_t chunk = (k.n + kClBlocks - 1) / kClBlocks;
     return chunk <= (int64_t)kClMaxU[bicgstab] * kClThreads && cl_smem(chunk, k.width) <= (size_t)kClSmemMax &&

@@ -4619,8 +4619,12 @@ static int launch_split_m(const gf_krylov_t* k, void* stream) {
         return launch_split_rows<BoxRows<double, false, false, int>, MINB, PAIRS, QREC, XA, PFA, PFB>(
             k, BoxRows<double, false, false, int>{k->val, (int)k->n, (int)k->stride_y, (int)k->stride_z}, st);
     }
-    // One slot at a time (the loop of a plain SpMV): the occupancy, not the
-    // loads of one thread, keeps the memory system busy.
+    // Rows of exactly six slots are unrolled by the compiler, so GRP is left at
+    // one.  The forms with four blocks an SM were tuned on an octree's rows and
+    // are the faster here too (variant 29, us an iteration, with eight blocks
+    // and single prefetches before in brackets): off a box 51.9 (67.7) at
+    // 1.33M cells, 74.4 (88.3) at 2.10M, 132.2 (146.7) at 4.10M; boxes that
+    // are not symmetric 45.1 (60.7), 61.8 (78.1), 113.5 (127.1).
     if (k->width == 6)
         return launch_split_rows<EllRows<double, 6, int, 1>, MINB, PAIRS, QREC, XA, PFA, PFB>(
             k, EllRows<double, 6, int, 1>{k->val, k->nbr, (int)k->n, k->width, k->row_len}, st);

@@ -1,6 +1,7 @@
 // Jacobi-PCG with the whole system resident on the grid's SMs (sm_100a).
 //
-// Beyond a cluster (gf_cluster.cu), up to about 425K cells, a system's rows
+// Beyond a cluster (gf_cluster.cu), up to 405,224 cells on 148 SMs (2,738 a
+// block; octrees, with two further entries a cell, 311,688), a system's rows
 // still fit the shared memory of all SMs together (80 bytes a cell: six
 // coefficients, six neighbour codes and the block's own part of z) and its
 // vectors their registers.  So an iteration touches global memory only for

@@ -45,7 +45,7 @@ VARIANTS = {
     8: "1024 threads, shared-memory vectors, q = A z + beta q recurrence, 1 cell/pass",
     9: "1024 threads, shared-memory vectors, q = A z + beta q recurrence, 2 cells/pass",
     10: "1024 threads, shared-memory vectors, one grid reduction and a halo sync per iteration, 1 cell/pass (FP32-inner: same form); "
-        "FP64 up to ~43K cells: the same form on one thread-block cluster, up to ~400K with the rows in shared memory too",
+        "FP64 up to ~45K cells: the same form on one thread-block cluster, up to ~400K with the rows in shared memory too",
     11: "1024 threads, shared-memory vectors, one grid reduction and a halo sync per iteration, 2 cells/pass",
     12: "512 threads x 2 a SM, vectors in global memory, q = A z + beta q recurrence (any size, FP64)",
     13: "1024 threads, vectors in global memory, q = A z + beta q recurrence (any size, FP64)",

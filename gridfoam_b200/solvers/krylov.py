@@ -49,7 +49,7 @@ def _split_graph_loop() -> bool:
 def default_variant(n: int, mixed: bool, symmetric: bool, box: bool = True) -> int:
     """CG launch shape by system size, from fixed-iteration timings on B200
     (``python -m gridfoam_b200.solvers.autotune``).  FP64 up to ~400K cells:
-    one reduction per iteration, up to ~43K cells on one thread-block cluster
+    one reduction per iteration, up to ~45K cells on one thread-block cluster
     with everything on the chip (2.1 against 6.4 us an iteration at 16^3, 4.0
     against 6.7 at 32^3), above that on the grid with a halo sync between
     neighbouring blocks, rows in shared memory and vectors in registers (6.1

@@ -353,10 +353,11 @@ int gf_split_loop_unroll(void);
  * up to 16 independent cases in ONE cooperative launch (CG: FP64 or, with
  * mixed = 1, FP32 inner iterations in FP64 refinement; BiCGStab: FP64).  System i
  * runs on blocks[i] persistent blocks of its own with its own workspace and
- * statistics, exactly as gf_pcg_solve / gf_bicgstab_solve run it on a grid
- * of blocks[i] blocks (register kernel, 256 threads a block for CG, 512 for
- * BiCGStab), so its result does not depend on the other systems in the
- * batch.  The block counts must fit on the device at once
+ * statistics (register kernels, 256 threads a block for CG, 512 for
+ * BiCGStab; the CG is the one gf_pcg_solve runs as variant 0 on a grid of
+ * blocks[i] blocks, the BiCGStab sums in another order than
+ * gf_bicgstab_solve's), so its result does not depend on the other systems
+ * in the batch.  The block counts must fit on the device at once
  * (gf_batch_max_blocks); CG systems have ncomp 1, BiCGStab systems share
  * one ncomp.  Two launches: a reset of the control blocks, then the solves. */
 int gf_pcg_solve_batched(const gf_krylov_t* systems, int32_t count,
