@@ -127,11 +127,12 @@ __device__ __forceinline__ void bicgstab_body(const gf_krylov_t& K, int bk, int 
         ok = grid_sum<2 * NC>(sh, ctl, partials, loc, nmask);
         if (me < NC) {
             BiState& b = st[me];
-            const double r0 = norm_fin(sh.total[me], linf);
+            // a wait that ran out leaves no totals
+            const double r0 = ok ? norm_fin(sh.total[me], linf) : no_value();
             b.r0 = r0;
             b.final = r0;
             b.thresh = fmax(K.atol, K.rtol * r0);
-            b.rho_old = sh.hh[me] = sh.total[NC + me];
+            b.rho_old = sh.hh[me] = ok ? sh.total[NC + me] : 0.0;
             b.restarts = 0;
             b.its = 0;
             b.converged = 0;

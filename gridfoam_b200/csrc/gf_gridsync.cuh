@@ -57,8 +57,9 @@ __device__ __forceinline__ bool grid_sync(GridShared<T, NVMAX>& sh, KCtl* ctl) {
 }
 
 // Sums over all blocks of NV values a thread (max where maxmask has the bit
-// set), and the barrier.  The totals are left in total; every block adds
-// the blocks' partials in the same fixed order.
+// set), and the barrier.  The totals are left in total (what was there before
+// stays when the wait gave up); every block adds the blocks' partials in the
+// same fixed order.
 template <int NV, int T, int NVMAX>
 __device__ __forceinline__ bool grid_sum(GridShared<T, NVMAX>& sh, KCtl* ctl, double* partials, double (&v)[NV], unsigned maxmask) {
     constexpr int kSlots = GridShared<T, NVMAX>::kSlots, kPer = kSlots / 32, kLoads = 5;

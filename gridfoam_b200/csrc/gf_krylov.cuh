@@ -37,9 +37,12 @@ __device__ __forceinline__ unsigned long long load_acquire(const unsigned long l
     return v;
 }
 
+// NaN: what a reduction that timed out has in place of its sums.
+__device__ __forceinline__ double no_value() { return __longlong_as_double(0x7ff8000000000000LL); }
+
 // Maximum that keeps a NaN (a norm with one must not pass a stopping test).
 __device__ __forceinline__ double nmax(double a, double b) {
-    if (a != a || b != b) return __longlong_as_double(0x7ff8000000000000LL);
+    if (a != a || b != b) return no_value();
     return fmax(a, b);
 }
 

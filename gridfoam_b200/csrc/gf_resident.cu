@@ -220,9 +220,10 @@ __global__ void __launch_bounds__(kRT, 1) k_pcg_resident(gf_krylov_t K, int chun
     atomicMin(&s_lo, lo);
     atomicMax(&s_hi, hi);
     bool ok = grid_sum<2>(sh, ctl, partials, loc, linf ? 1u : 0u);
-    const double r0 = norm_fin(sh.total[0], linf), thresh = fmax(K.atol, K.rtol * r0);
-    double fin = r0, rz = sh.total[1], alpha = 1.0;
-    int its = 0, status = r0 < thresh ? GF_OK : (!isfinite(r0) ? GF_NONFINITE : -1);
+    // (a wait that ran out leaves no totals)
+    const double r0 = ok ? norm_fin(sh.total[0], linf) : no_value(), thresh = fmax(K.atol, K.rtol * r0);
+    double fin = r0, rz = ok ? sh.total[1] : 0.0, alpha = 1.0;
+    int its = 0, status = !ok ? -1 : (r0 < thresh ? GF_OK : (!isfinite(r0) ? GF_NONFINITE : -1));
     if (K.max_iter <= 0 && status < 0) status = GF_MAX_ITER;
     // Every thread holds the same scalars (from the same totals) and takes
     // the same branches.
