@@ -83,11 +83,11 @@ class GfMesh(ctypes.Structure):
         ("reg_level", P),
         ("irr_cells", P),
         ("hang_cells", P),
-        ("n_irr", I64),
-        ("n_hang_cells", I64),
+        ("n_irr", I32),
+        ("n_hang_cells", I32),
         ("reg_h", F64 * 3),
-        ("stride_y", I64),
-        ("stride_z", I64),
+        ("stride_y", I32),
+        ("stride_z", I32),
     ]
 
 
@@ -280,32 +280,21 @@ class GfError(RuntimeError):
     """A gridfoam_b200 library call failed."""
 
 
-def _grad_launches(args) -> int:
-    """A gradient's launches, asked once a mesh descriptor (``args[0]`` is a
-    ``byref`` of it)."""
-    m = args[0]._obj
-    n = getattr(m, "grad_launches", 0)
-    if not n:
-        n = m.grad_launches = load().gf_lsq_grad_launches(args[0])
-    return n
+def _mesh_launches(m: GfMesh) -> dict:
+    """Launches of the calls whose kernels depend on the mesh, asked once a
+    mesh descriptor and kept on it."""
+    grad = load().gf_lsq_grad_launches(ctypes.byref(m))
+    m.launches = {"gf_lsq_grad": grad, "gf_lsq_grad_hang": int(m.n_hang_cells > 0) if m.hang_cells else grad,
+                  # axis-aligned internal faces and the boundary faces apart, or all in one
+                  "gf_face_flux": 1 + int(bool(m.face_axis) and m.n_faces > 0 and m.n_bnd > 0)}
+    return m.launches
 
 
-def _hang_grad_launches(args) -> int:
-    m = args[0]._obj
-    return int(m.n_hang_cells > 0) if m.hang_cells else _grad_launches(args)
-
-
-def _face_flux_launches(args) -> int:
-    """Axis-aligned internal faces and the boundary faces apart, or all in one."""
-    m = args[0]._obj
-    return 1 + int(bool(m.face_axis) and m.n_faces > 0 and m.n_bnd > 0)
-
-
-# Kernels launched per entry point (for launch accounting): a number, or a
-# function of the call's arguments.
+# Kernels launched per entry point (for launch accounting); 0: by the mesh
+# (the first argument, a ``byref`` of it).
 _LAUNCHES_PER_CALL = {"gf_fixed_values": 3, "gf_close_fixed_flux": 2, "gf_field_residual": 2, "gf_continuity_sums": 2,
-                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2, "gf_lsq_grad": _grad_launches,
-                      "gf_lsq_grad_hang": _hang_grad_launches, "gf_face_flux": _face_flux_launches}
+                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2, "gf_lsq_grad": 0, "gf_lsq_grad_hang": 0,
+                      "gf_face_flux": 0}
 LAUNCHES: collections.Counter = collections.Counter()
 # Launches known only after the device ran (the split CG's graph loop, whole
 # bodies of some iterations): callables giving their counts, kept while
@@ -329,7 +318,10 @@ def call(name: str, *args) -> int:
     lib = load()
     status = getattr(lib, name)(*args)
     per = _LAUNCHES_PER_CALL.get(name, 1)
-    LAUNCHES[name] += per if per.__class__ is int else per(args)
+    if per == 0:
+        m = args[0]._obj
+        per = (getattr(m, "launches", None) or _mesh_launches(m))[name]
+    LAUNCHES[name] += per
     if status != GF_OK:
         msg = lib.gf_last_error().decode(errors="replace")
         raise GfError(f"{name} failed with status {status}: {msg}")
