@@ -213,6 +213,7 @@ _SIGNATURES = {
     "gf_split_loop_unroll": ([], ctypes.c_int),
     "gf_rau_hbya": ([P, I32, P, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_simplec_rAtU": ([P, P, P, P, P], ctypes.c_int),
+    "gf_face_flux_launches": ([P, I32], ctypes.c_int),
     "gf_face_flux": ([P, I32, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_fvc_div": ([P, I32, P, P, P], ctypes.c_int),
     "gf_reconstruct": ([P, P, P, P], ctypes.c_int),
@@ -285,8 +286,8 @@ def _mesh_launches(m: GfMesh) -> dict:
     mesh descriptor and kept on it."""
     grad = load().gf_lsq_grad_launches(ctypes.byref(m))
     m.launches = {"gf_lsq_grad": grad, "gf_lsq_grad_hang": int(m.n_hang_cells > 0) if m.hang_cells else grad,
-                  # axis-aligned internal faces and the boundary faces apart, or all in one
-                  "gf_face_flux": 1 + int(bool(m.face_axis) and m.n_faces > 0 and m.n_bnd > 0)}
+                  # a gradient is passed where there are hanging faces
+                  "gf_face_flux": load().gf_face_flux_launches(ctypes.byref(m), int(m.n_hang > 0))}
     return m.launches
 
 

@@ -1546,6 +1546,20 @@ __global__ void __launch_bounds__(256, DDT ? 3 : 4) k_face_flux_axis(gf_mesh_t m
     }
 }
 
+// Internal faces in a kernel of their own (k_face_flux_axis), the boundary
+// faces in a second one.  With hanging faces (a gradient) only from 640K faces
+// on: below, the second launch costs a launch-bound pass more than the kernel
+// gains (a pass of explicit operators on octrees, one kernel and two: 315K
+// faces 171 and 174 us, 546K 171 and 173, 830K 176 and 172, 1.10M 189 and 179;
+// the flux alone on the device 5.9 and 5.2, 8.6 and 6.3, 12.1 and 6.9, 20 and
+// 10).  Both give the same bits.
+constexpr int64_t kAxisHangFaces = 655360;
+
+static bool flux_by_axis(const gf_mesh_t* m, bool gradient) {
+    return m->face_axis != nullptr && m->n_faces > 0 && m->n_faces < (int64_t)INT32_MAX &&
+           (!gradient || m->n_faces >= kAxisHangFaces);
+}
+
 // Two rows of the extended face layout a thread and pass: their indices,
 // then every gather, before any is used (one row at a time with a loop over
 // the components was a chain of dependent loads at 2.7-2.9 TB/s).  4.08M-cell
@@ -2150,6 +2164,10 @@ int gf_simplec_rAtU(const gf_mesh_t* m, const double* rau, const double* h1, dou
     return check_launch("gf_simplec_rAtU");
 }
 
+int gf_face_flux_launches(const gf_mesh_t* m, int32_t gradient) {
+    return m != nullptr && flux_by_axis(m, gradient != 0) && m->n_bnd > 0 ? 2 : 1;
+}
+
 int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel, const int8_t* u_kind, const double* u_psib,
                  const gf_ddtcorr_t* ddt, const double* grad_vel, double* phi, void* stream) {
     if (!valid_mesh(m) || (mode != 0 && mode != 1) || vel == nullptr || u_kind == nullptr) {
@@ -2168,7 +2186,7 @@ int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel, const int8
         }
     }
     cudaStream_t st = GF_STREAM(stream);
-    if (m->face_axis != nullptr && m->n_faces > 0 && m->n_faces < (int64_t)INT32_MAX) {
+    if (flux_by_axis(m, grad_vel != nullptr)) {
         const unsigned g = grid_for((m->n_faces + 1) / 2);
         auto kern = grad_vel != nullptr ? (has ? k_face_flux_axis<true, true> : k_face_flux_axis<false, true>)
                                         : (has ? k_face_flux_axis<true, false> : k_face_flux_axis<false, false>);

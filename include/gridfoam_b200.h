@@ -405,6 +405,8 @@ int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel,
                  const int8_t* u_kind, const double* u_psib,
                  const gf_ddtcorr_t* ddt, const double* grad_vel, double* phi,
                  void* stream);
+/* Kernels that it launches on this mesh, with a velocity gradient or without. */
+int gf_face_flux_launches(const gf_mesh_t* m, int32_t gradient);
 
 /* fv/fvc/reconstruct.py:28-117: cell velocity U [3][C] from the face flux
  * phi (extended layout [F | Nb]): (sum |Sf| n n^T)^-1 sum n phi over every
