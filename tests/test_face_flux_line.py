@@ -20,11 +20,10 @@ LINE = 655360  # internal faces
 @pytest.mark.parametrize("size,kernels", [((40, 27, 5), 1), ((92, 60, 12), 1), ((96, 62, 12), 2), ((116, 74, 14), 2)])
 @pytest.mark.parametrize("ddt", [False, True])
 def test_octree_face_flux(size, kernels, ddt):
-    from torch.profiler import ProfilerActivity, profile
-
     from gridfoam_b200._lib import GfDdtCorr, GfMesh, call, ptr, stream_ptr
     from gridfoam_b200.core.field import CellField, FaceField
     from gridfoam_b200.fv.fvc import _eval_state, _hanging_grad
+    from tests.profiled import record
 
     grid = _grid("wake", size)
     F = grid.num_internal_faces
@@ -45,14 +44,17 @@ def test_octree_face_flux(size, kernels, ddt):
     general = GfMesh()
     ctypes.pointer(general)[0] = grid.cmesh
     general.face_axis = None
-    out = []
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
+
+    def run():
+        out = []
         for m in (general, grid.cmesh):
             phi = FaceField(grid, "phi")
             phi.store.fill_(float("nan"))
             call("gf_face_flux", ctypes.byref(m), 0, ptr(U.store), ptr(t.kind), ptr(t.psib),
                  None if d is None else ctypes.byref(d), ptr(grad), ptr(phi.store), stream_ptr())
             out.append(phi.store)
-        torch.cuda.synchronize()
+        return out
+
+    out, events = record(run)
     assert not bool(out[0].isnan().any()) and torch.equal(out[0], out[1])
-    assert sum(e.count for e in prof.key_averages() if "k_face_flux" in e.key) == 1 + kernels
+    assert sum(n for key, n in events if "k_face_flux" in key) == 1 + kernels

@@ -25,17 +25,16 @@ def _grid(mesh, size):
 
 def _kernels(run):
     """The package's kernels launched by ``run``, by the profiler and by the account."""
-    from torch.profiler import ProfilerActivity, profile
-
     from gridfoam_b200 import _lib
+    from tests.profiled import record
+
+    def counted():
+        _lib.clear_launches()
+        run()
 
     run()
-    torch.cuda.synchronize()
-    _lib.clear_launches()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        run()
-        torch.cuda.synchronize()
-    return sum(e.count for e in prof.key_averages() if "gf::k_" in e.key), _lib.launch_total()
+    _, events = record(counted)
+    return sum(n for key, n in events if "gf::k_" in key), _lib.launch_total()
 
 
 @pytest.mark.parametrize("mesh,size", [("box", (20, 21, 22)), ("box", (72, 71, 70)), ("wake", (40, 27, 5)),

@@ -19,13 +19,10 @@ SIX = r"k_pcg_resident(<6, true>|ILi6ELb1E)"  # the name as written or as linked
 
 
 def _ran(run):
-    from torch.profiler import ProfilerActivity, profile
+    from tests.profiled import record
 
-    torch.cuda.synchronize()
-    with profile(activities=[ProfilerActivity.CUDA]) as prof:
-        out = run()
-        torch.cuda.synchronize()
-    return out, " ".join(e.key for e in prof.key_averages())
+    out, events = record(run)
+    return out, " ".join(key for key, _ in events)
 
 
 # cells, block cap, wide rows: six cells a thread (chunks of 2,049 to 2,106
