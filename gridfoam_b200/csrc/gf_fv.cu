@@ -29,6 +29,7 @@ template <int nc>
 __global__ void __launch_bounds__(128) k_bc_state(gf_mesh_t m, gf_bc_t bc, const double* __restrict__ psi,
                                                   gf_bc_aux_t aux, gf_bc_state_t out) {
     const int64_t nb = m.n_bnd;
+    const int64_t vs = bc.reserved ? 0 : nb;  // see gf_bc_state
     const int64_t C = m.n_cells;
     for (int64_t b = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; b < nb;
          b += (int64_t)gridDim.x * blockDim.x) {
@@ -38,8 +39,7 @@ __global__ void __launch_bounds__(128) k_bc_state(gf_mesh_t m, gf_bc_t bc, const
         double psiP[3], value[3], refv[3] = {0, 0, 0}, refg[3] = {0, 0, 0};
 #pragma unroll
         for (int k = 0; k < nc; ++k) {
-            // before the kind is known; a table of kinds that need none may have none
-            value[k] = bc.value != nullptr ? __ldg(bc.value + k * nb + b) : 0.0;
+            value[k] = __ldg(bc.value + k * vs + b);  // before the kind is known
             psiP[k] = psi[k * C + c];
         }
         double frac = 0.0;
@@ -1983,8 +1983,14 @@ int gf_bc_state(const gf_mesh_t* m, const gf_bc_t* bc, const double* psi, const 
     if (!valid_nc(bc->ncomp)) return GF_ERR_INVALID;
     if (m->n_bnd == 0) return GF_OK;
     gf_bc_aux_t a = aux ? *aux : gf_bc_aux_t{nullptr, nullptr, nullptr, nullptr, nullptr};
+    // The kernel reads a value before it knows the face's kind.  A table of
+    // kinds that need none may have no values: any row of faces serves then
+    // (a test of the pointer at each load cost 0.7 us of 7.2 on 230K faces).
+    gf_bc_t t = *bc;
+    t.reserved = t.value == nullptr;
+    if (t.value == nullptr) t.value = m->bnd_mag_d;
     auto kern = bc->ncomp == 1 ? k_bc_state<1> : k_bc_state<3>;
-    kern<<<grid_for(m->n_bnd, 128), 128, 0, GF_STREAM(stream)>>>(*m, *bc, psi, a, *out);
+    kern<<<grid_for(m->n_bnd, 128), 128, 0, GF_STREAM(stream)>>>(*m, t, psi, a, *out);
     return check_launch("gf_bc_state");
 }
 
