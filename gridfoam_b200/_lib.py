@@ -195,7 +195,6 @@ _SIGNATURES = {
     "gf_krylov_workspace_size": ([I64, I32, I32], I64),
     "gf_bc_state": ([P, P, P, P, P, P], ctypes.c_int),
     "gf_lsq_grad": ([P, I32, P, P, P, P, P], ctypes.c_int),
-    "gf_lsq_grad_launches": ([P], ctypes.c_int),
     "gf_lsq_grad_hang": ([P, I32, P, P, P, P, P], ctypes.c_int),
     "gf_assemble": ([P, P, P], ctypes.c_int),
     "gf_momentum_finalize": ([P, I32, F64, P, P, P, P, P, P], ctypes.c_int),
@@ -213,7 +212,7 @@ _SIGNATURES = {
     "gf_split_loop_unroll": ([], ctypes.c_int),
     "gf_rau_hbya": ([P, I32, P, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_simplec_rAtU": ([P, P, P, P, P], ctypes.c_int),
-    "gf_face_flux_launches": ([P, I32], ctypes.c_int),
+    "gf_further_launches": ([], I64),
     "gf_face_flux": ([P, I32, P, P, P, P, P, P, P], ctypes.c_int),
     "gf_fvc_div": ([P, I32, P, P, P], ctypes.c_int),
     "gf_reconstruct": ([P, P, P, P], ctypes.c_int),
@@ -281,22 +280,13 @@ class GfError(RuntimeError):
     """A gridfoam_b200 library call failed."""
 
 
-def _mesh_launches(m: GfMesh) -> dict:
-    """Launches of the calls whose kernels depend on the mesh, asked once a
-    mesh descriptor and kept on it."""
-    grad = load().gf_lsq_grad_launches(ctypes.byref(m))
-    m.launches = {"gf_lsq_grad": grad, "gf_lsq_grad_hang": int(m.n_hang_cells > 0) if m.hang_cells else grad,
-                  # a gradient is passed where there are hanging faces
-                  "gf_face_flux": load().gf_face_flux_launches(ctypes.byref(m), int(m.n_hang > 0))}
-    return m.launches
-
-
-# Kernels launched per entry point (for launch accounting); 0: by the mesh
-# (the first argument, a ``byref`` of it).
+# Kernels launched per entry point (for launch accounting).  Second kernels
+# that depend on the mesh are counted by the library (gf_further_launches), at
+# no cost to a call.
 _LAUNCHES_PER_CALL = {"gf_fixed_values": 3, "gf_close_fixed_flux": 2, "gf_field_residual": 2, "gf_continuity_sums": 2,
-                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2, "gf_lsq_grad": 0, "gf_lsq_grad_hang": 0,
-                      "gf_face_flux": 0}
+                      "gf_pcg_solve_batched": 2, "gf_bicgstab_solve_batched": 2}
 LAUNCHES: collections.Counter = collections.Counter()
+_FURTHER_BEFORE = 0  # gf_further_launches at the last clear
 # Launches known only after the device ran (the split CG's graph loop, whole
 # bodies of some iterations): callables giving their counts, kept while
 # TRACK_DEFERRED is set (see ``launch_total``).
@@ -304,25 +294,28 @@ TRACK_DEFERRED = False
 DEFERRED_LAUNCHES: list = []
 
 
+def _further_launches() -> int:
+    return _LIB.gf_further_launches() if _LIB is not None else 0
+
+
 def clear_launches() -> None:
+    global _FURTHER_BEFORE
     LAUNCHES.clear()
     DEFERRED_LAUNCHES.clear()
+    _FURTHER_BEFORE = _further_launches()
 
 
 def launch_total() -> int:
     """Kernels launched since ``clear_launches`` (read after a synchronize)."""
-    return sum(LAUNCHES.values()) + sum(int(f()) for f in DEFERRED_LAUNCHES)
+    return (sum(LAUNCHES.values()) + _further_launches() - _FURTHER_BEFORE
+            + sum(int(f()) for f in DEFERRED_LAUNCHES))
 
 
 def call(name: str, *args) -> int:
     """Call ``name`` and raise :class:`GfError` on a non-zero status."""
     lib = load()
     status = getattr(lib, name)(*args)
-    per = _LAUNCHES_PER_CALL.get(name, 1)
-    if per == 0:
-        m = args[0]._obj
-        per = (getattr(m, "launches", None) or _mesh_launches(m))[name]
-    LAUNCHES[name] += per
+    LAUNCHES[name] += _LAUNCHES_PER_CALL.get(name, 1)
     if status != GF_OK:
         msg = lib.gf_last_error().decode(errors="replace")
         raise GfError(f"{name} failed with status {status}: {msg}")

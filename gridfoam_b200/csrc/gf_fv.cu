@@ -7,11 +7,15 @@
 // are written once, without atomics, and are bitwise reproducible.
 #include "gf_common.cuh"
 
+#include <atomic>
 #include <mutex>
 
 namespace gf {
 
 static thread_local std::string g_last_error;
+
+// Kernels launched beyond one a call (gf_further_launches).
+static std::atomic<int64_t> g_further_launches{0};
 
 void set_error(const char* fmt, ...) {
     char buf[512];
@@ -2005,6 +2009,7 @@ int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8
                                     : (ncomp == 1 ? k_lsq_regular<1, false> : k_lsq_regular<3, false>);
         kern<<<g, kThreads, 0, st>>>(*m, ih, psi, grad);
         lsq_list(m, ncomp, m->n_irr, m->irr_cells, psi, bc_kind, psib, grad, st);
+        if (m->n_irr > 0) ++g_further_launches;
         return check_launch("gf_lsq_grad");
     }
     const bool six = m->ell_width == 6 && m->n_faces < (int64_t)INT32_MAX;
@@ -2028,13 +2033,12 @@ int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8
     return check_launch("gf_lsq_grad");
 }
 
-int gf_lsq_grad_launches(const gf_mesh_t* m) { return m != nullptr && has_regular(m) && m->n_irr > 0 ? 2 : 1; }
-
 int gf_lsq_grad_hang(const gf_mesh_t* m, int32_t ncomp, const double* psi, const int8_t* bc_kind, const double* psib,
                      double* grad, void* stream) {
     if (!valid_mesh(m) || !valid_nc(ncomp) || m->lsq_ata_inv == nullptr) return GF_ERR_INVALID;
     if (m->hang_cells == nullptr || m->ell_width < 6 || m->n_faces >= (int64_t)INT32_MAX)
         return gf_lsq_grad(m, ncomp, psi, bc_kind, psib, grad, stream);
+    if (m->n_hang_cells <= 0) --g_further_launches;
     lsq_list(m, ncomp, m->n_hang_cells, m->hang_cells, psi, bc_kind, psib, grad, GF_STREAM(stream));
     return check_launch("gf_lsq_grad_hang");
 }
@@ -2170,9 +2174,7 @@ int gf_simplec_rAtU(const gf_mesh_t* m, const double* rau, const double* h1, dou
     return check_launch("gf_simplec_rAtU");
 }
 
-int gf_face_flux_launches(const gf_mesh_t* m, int32_t gradient) {
-    return m != nullptr && flux_by_axis(m, gradient != 0) && m->n_bnd > 0 ? 2 : 1;
-}
+int64_t gf_further_launches(void) { return g_further_launches; }
 
 int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel, const int8_t* u_kind, const double* u_psib,
                  const gf_ddtcorr_t* ddt, const double* grad_vel, double* phi, void* stream) {
@@ -2197,9 +2199,11 @@ int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel, const int8
         auto kern = grad_vel != nullptr ? (has ? k_face_flux_axis<true, true> : k_face_flux_axis<false, true>)
                                         : (has ? k_face_flux_axis<true, false> : k_face_flux_axis<false, false>);
         kern<<<g, kThreads, 0, st>>>(*m, vel, d, grad_vel, phi);
-        if (m->n_bnd > 0)
+        if (m->n_bnd > 0) {
             k_face_flux<<<grid_for(m->n_bnd), kThreads, 0, st>>>(*m, mode, vel, u_kind, u_psib, d, has, grad_vel,
                                                                   phi, m->n_faces);
+            ++g_further_launches;
+        }
     } else {
         k_face_flux<<<grid_for(m->n_faces + m->n_bnd), kThreads, 0, st>>>(*m, mode, vel, u_kind, u_psib, d, has,
                                                                           grad_vel, phi, 0);

@@ -277,8 +277,6 @@ int gf_bc_state(const gf_mesh_t* m, const gf_bc_t* bc, const double* psi,
 int gf_lsq_grad(const gf_mesh_t* m, int32_t ncomp, const double* psi,
                 const int8_t* bc_kind, const double* psib, double* grad,
                 void* stream);
-/* Kernels that gf_lsq_grad launches on this mesh. */
-int gf_lsq_grad_launches(const gf_mesh_t* m);
 
 /* The same gradient at the cells with a hanging face only (mesh hang_cells;
  * everywhere when that is NULL): all that the hanging-face corrections of
@@ -405,8 +403,10 @@ int gf_face_flux(const gf_mesh_t* m, int32_t mode, const double* vel,
                  const int8_t* u_kind, const double* u_psib,
                  const gf_ddtcorr_t* ddt, const double* grad_vel, double* phi,
                  void* stream);
-/* Kernels that it launches on this mesh, with a velocity gradient or without. */
-int gf_face_flux_launches(const gf_mesh_t* m, int32_t gradient);
+/* Kernels that gf_lsq_grad, gf_lsq_grad_hang and gf_face_flux have launched
+ * beyond one a call (they take a second one by the mesh), since the library
+ * was loaded. */
+int64_t gf_further_launches(void);
 
 /* fv/fvc/reconstruct.py:28-117: cell velocity U [3][C] from the face flux
  * phi (extended layout [F | Nb]): (sum |Sf| n n^T)^-1 sum n phi over every
