@@ -259,7 +259,8 @@ class AxisProjectedGrid:
         owner, neighbour, axis, C = self._owner, self._neighbour, self._axis, self._num_cells
         center, sizes = self.dev["center"], self._cell_sizes
         h = sizes.amin(0)
-        level = torch.round(torch.log2(sizes[:, 0] / h[0])).clamp(0, 32).long()
+        # (a size that is zero, negative or not a number has no level: 32)
+        level = torch.nan_to_num(torch.log2(sizes[:, 0] / h[0]), nan=32.0).round().clamp(0, 32).long()
         scale = torch.tensor([2.0**i for i in range(33)], dtype=torch.float64, device=sizes.device)[level]
         ok = (level < 32) & (sizes == h * scale[:, None]).all(1)
         want = h[axis] * scale[owner]

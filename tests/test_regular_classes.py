@@ -48,3 +48,22 @@ def test_regular_cells_match_the_restatement(name):
     assert grid.cmesh.n_irr == int((want == 255).sum())
     if name == "wake":
         assert {0, 2, 255} <= set(want.tolist())  # the finest and the coarsest level have regular cells
+
+
+@pytest.mark.filterwarnings("ignore::RuntimeWarning")
+@pytest.mark.parametrize("value,whole_axis", [(0.0, False), (-1.0, False), (float("nan"), False), (float("inf"), False),
+                                              (0.0, True), (-1.0, True)])
+def test_sizes_without_a_level_are_not_regular(value, whole_axis):
+    """A mesh with such sizes was accepted before there were classes."""
+    from gridfoam_b200.cases import build_mesh, cavity_case
+    from gridfoam_b200.core.grid import AxisProjectedGrid
+    from gridfoam_b200.meta.config import SimulatorConfig
+
+    case = cavity_case(5)
+    mesh = build_mesh(case["mesh"], device="cpu")
+    sizes = np.array(mesh.cell_sizes, dtype=np.float64)
+    cells = slice(None) if whole_axis else [62]  # the middle cell
+    sizes[cells, 0] = value
+    mesh.cell_sizes = sizes
+    grid = AxisProjectedGrid(SimulatorConfig.model_validate(case["simulator"]), mesh, device="cpu")
+    assert (grid.dev["reg_level"].numpy()[cells] == 255).all()
