@@ -18,11 +18,15 @@ pytestmark = pytest.mark.gpu
 SIX = r"k_pcg_resident(<6, true>|ILi6ELb1E)"  # the name as written or as linked
 
 
-def _ran(run):
-    from tests.profiled import record
+def _ran(run, form):
+    """``run``'s result and whether a kernel of the form ran."""
+    from tests.profiled import lost, record
 
-    out, events = record(run)
-    return out, " ".join(key for key, _ in events)
+    names = lambda events: " ".join(key for key, _ in events if "gf::k_" in key or "_ZN2gf" in key)  # noqa: E731
+    out, events = record(run, lambda events: re.search(form, names(events)))
+    if not names(events):
+        lost()
+    return out, names(events)
 
 
 # cells, block cap, wide rows: six cells a thread (chunks of 2,049 to 2,106
@@ -35,7 +39,7 @@ def test_resident_cg_of_six_cells_a_thread_with_wide_rows(n, cap, form, reach, l
     s, diag, val = _ring(n, reach, long_every)
     g = torch.Generator(device="cuda").manual_seed(5)
     rhs = torch.randn((1, n), dtype=torch.float64, device="cuda", generator=g)
-    (x, st), kernels = _ran(lambda: _solve(s, diag, val, rhs, 10, cap))
+    (x, st), kernels = _ran(lambda: _solve(s, diag, val, rhs, 10, cap), form)
     assert re.search(form, kernels), kernels
     ref, st_ref = _solve(s, diag, val, rhs, 0, 148)
     assert st.status == st_ref.status == "ok"
@@ -52,7 +56,7 @@ def test_cluster_cg_at_its_largest_system(shape, form, layout):
     s = _system(shape, layout)
     g = torch.Generator(device="cuda").manual_seed(7)
     rhs = torch.randn((1, s.num_cells), dtype=torch.float64, device="cuda", generator=g)
-    (x, st), kernels = _ran(lambda: solve(s, "cg", rhs, False, "l_2", layout))
+    (x, st), kernels = _ran(lambda: solve(s, "cg", rhs, False, "l_2", layout), form)
     assert re.search(form, kernels), kernels
     ref, st_ref = solve(s, "cg", rhs, True, "l_2", layout)
     assert st[0].status == st_ref[0].status == "ok"
